@@ -162,6 +162,10 @@ EXPORTED = (
     "cvlbm_fno_to_bf16",
     "cvlbm_fno_mse",
     "cvlbm_fno_adam",
+    "cvlbm_fno_layer_fwd",
+    "cvlbm_fno_layer_bwd",
+    "cvlbm_fno_mse_mean",
+    "cvlbm_fno_adam_list",
 )
 
 
@@ -232,6 +236,11 @@ def load(require_cuda: bool = True):
         "cvlbm_fno_spec_mix_bwd": (i32, [i32, i32, i32, pI, pI, pI, pI, pI, pI]),
         "cvlbm_fno_to_bf16": (i32, [i64, pI, pI, pI]),
         "cvlbm_fno_mse": (i32, [i32, i32, i32, pI, pI, pI, pI, C.c_float, pI, pI, i32, pI]),
+        "cvlbm_fno_layer_fwd": (i32, [i32, i32, i32, i32, pI, pI, pI, pI, i32, pI, pI, pI, pI]),
+        "cvlbm_fno_layer_bwd": (i32, [i32, i32, i32, i32, pI, pI, pI, pI, pI, pI, pI, pI, pI, pI]),
+        "cvlbm_fno_mse_mean": (i32, [i32, i32, i32, pI, pI, pI, pI, pI, pI, pI, i32, pI]),
+        "cvlbm_fno_adam_list": (i32, [i32, pI, pI, pI, pI, pI, C.c_float, C.c_float, C.c_float,
+                                      C.c_float, pI]),
         "cvlbm_fno_adam": (i32, [i64, pI, pI, pI, pI, C.c_float, C.c_float, C.c_float,
                                  C.c_float, pI]),
     }

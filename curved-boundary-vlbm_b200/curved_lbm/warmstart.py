@@ -27,6 +27,7 @@ library's CUDA-core kernels.  Weights are fp32.
 
 from __future__ import annotations
 
+import ctypes as C
 import math
 import time as _time
 
@@ -116,32 +117,27 @@ class FNO:
                                                 _native.ptr(self._ws), self._ws.numel() * 4,
                                                 self._s()), "cvlbm_gemm_bf16")
 
-    def _bf16(self, x):
-        import torch
-
-        out = torch.empty(x.shape, dtype=torch.bfloat16, device=self.dev)
-        _native.check(self._lib.cvlbm_fno_to_bf16(x.numel(), _native.ptr(x), _native.ptr(out),
-                                                  self._s()), "cvlbm_fno_to_bf16")
-        return out
-
-    def _pw(self, x, W, b, s=None, act=0, keep_z=False):
+    def _pw(self, x, W, b, s=None, act=0, keep_z=False, bf16=False):
+        """(y, z, y in bf16) of one pointwise layer; z and the bf16 copy on request."""
         import torch
 
         Cout, Cin = W.shape
         y = torch.empty((self.B, Cout, self.G), dtype=torch.float32, device=self.dev)
         z = torch.empty_like(y) if keep_z else None
-        _native.check(self._lib.cvlbm_fno_pointwise_fwd(
+        yb = (torch.empty((self.B * Cout, self.G), dtype=torch.bfloat16, device=self.dev)
+              if bf16 else None)
+        _native.check(self._lib.cvlbm_fno_layer_fwd(
             self.B, self.G, Cin, Cout, _native.ptr(x), _native.ptr(W), _native.ptr(b),
-            _native.ptr(s), act, _native.ptr(z), _native.ptr(y), self._s()),
-            "cvlbm_fno_pointwise_fwd")
-        return y, z
+            _native.ptr(s), act, _native.ptr(z), _native.ptr(y), _native.ptr(yb), self._s()),
+            "cvlbm_fno_layer_fwd")
+        return y, z, yb
 
-    def _pw_bwd(self, dz, x, W, dW, db, dx=None, accumulate=0):
+    def _pw_bwd(self, dy, x, W, dW, db, z=None, dx=None, dzb=None):
         Cout, Cin = W.shape
-        _native.check(self._lib.cvlbm_fno_pointwise_bwd(
-            self.B, self.G, Cin, Cout, _native.ptr(dz), _native.ptr(x), _native.ptr(W),
-            _native.ptr(dx), accumulate, _native.ptr(dW), _native.ptr(db),
-            _native.ptr(self._scratch), self._s()), "cvlbm_fno_pointwise_bwd")
+        _native.check(self._lib.cvlbm_fno_layer_bwd(
+            self.B, self.G, Cin, Cout, _native.ptr(dy), _native.ptr(z), _native.ptr(x),
+            _native.ptr(W), _native.ptr(dx), _native.ptr(dzb), _native.ptr(dW), _native.ptr(db),
+            _native.ptr(self._scratch), self._s()), "cvlbm_fno_layer_bwd")
 
     # -- forward / backward ------------------------------------------------------
     def forward(self, x):
@@ -150,9 +146,8 @@ class FNO:
 
         P, B, C, G, M = self.params, self.B, self.C, self.G, self.M
         cache = {"x": x}
-        h, _ = self._pw(x, P["W0"], P["b0"])
+        h, _, hb = self._pw(x, P["W0"], P["b0"], bf16=self.L > 0)
         for l in range(1, self.L + 1):
-            hb = self._bf16(h).view(B * C, G)
             a = torch.empty((B * C, M), dtype=torch.float32, device=self.dev)
             self._gemm(hb, self.phiT, a)  # a = h Phi
             bh = torch.empty((B * C, M), dtype=torch.bfloat16, device=self.dev)
@@ -163,11 +158,13 @@ class FNO:
             s = torch.empty((B * C, G), dtype=torch.float32, device=self.dev)
             self._gemm(bh, self.phi, s)  # s = bh Phi^T
             act = 1 if l < self.L else 0
-            hn, z = self._pw(h, P[f"W{l}"], P[f"b{l}"], s=s, act=act, keep_z=True)
+            # the last layer has no activation (its z is h) and no transform after it
+            hn, z, hb = self._pw(h, P[f"W{l}"], P[f"b{l}"], s=s, act=act, keep_z=act == 1,
+                                 bf16=l < self.L)
             cache[l] = (h, a, z)
             h = hn
         cache["h"] = h
-        y, _ = self._pw(h, P["Wp"], P["bp"])
+        y, _, _ = self._pw(h, P["Wp"], P["bp"])
         self._cache = cache
         return y
 
@@ -181,16 +178,10 @@ class FNO:
         self._pw_bwd(dy, cache["h"], P["Wp"], Gr["Wp"], Gr["bp"], dx=dh)
         for l in range(self.L, 0, -1):
             h, a, z = cache[l]
-            if l < self.L:
-                dz = torch.empty_like(dh)
-                _native.check(self._lib.cvlbm_fno_gelu_bwd(dh.numel(), _native.ptr(z),
-                                                           _native.ptr(dh), _native.ptr(dz),
-                                                           self._s()), "cvlbm_fno_gelu_bwd")
-            else:
-                dz = dh
             dprev = torch.empty((B, C, G), dtype=torch.float32, device=self.dev)
-            self._pw_bwd(dz, h, P[f"W{l}"], Gr[f"W{l}"], Gr[f"b{l}"], dx=dprev)
-            dzb = self._bf16(dz).view(B * C, G)
+            dzb = torch.empty((B * C, G), dtype=torch.bfloat16, device=self.dev)
+            # dz = dh * gelu'(z) (z None: no activation), its bf16 copy, W^T dz, dW, db
+            self._pw_bwd(dh, h, P[f"W{l}"], Gr[f"W{l}"], Gr[f"b{l}"], z=z, dx=dprev, dzb=dzb)
             dbh = torch.empty((B * C, M), dtype=torch.float32, device=self.dev)
             self._gemm(dzb, self.phiT, dbh)  # dbh = dz Phi
             da = torch.empty((B * C, M), dtype=torch.bfloat16, device=self.dev)
@@ -209,12 +200,13 @@ class FNO:
         n_parts = 256
         dy = torch.empty_like(y)
         part = torch.empty(n_parts, dtype=torch.float32, device=self.dev)
-        cnt = float(mask.sum().item()) * C_OUT
-        _native.check(self._lib.cvlbm_fno_mse(self.B, C_OUT, self.G, _native.ptr(y),
-                                              _native.ptr(t), _native.ptr(mask),
-                                              _native.ptr(wch), 1.0 / max(cnt, 1.0),
-                                              _native.ptr(dy), _native.ptr(part), n_parts,
-                                              self._s()), "cvlbm_fno_mse")
+        # mean over the masked entries; the mask's sum stays on the device
+        msum = mask.sum(dtype=torch.float32)
+        _native.check(self._lib.cvlbm_fno_mse_mean(self.B, C_OUT, self.G, _native.ptr(y),
+                                                   _native.ptr(t), _native.ptr(mask),
+                                                   _native.ptr(wch), _native.ptr(msum),
+                                                   _native.ptr(dy), _native.ptr(part), n_parts,
+                                                   self._s()), "cvlbm_fno_mse_mean")
         return part, dy
 
     def adam_step(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
@@ -226,12 +218,12 @@ class FNO:
         st = self._adam
         st["t"] += 1
         lr_t = lr * math.sqrt(1 - b2 ** st["t"]) / (1 - b1 ** st["t"])
-        for k, p in self.params.items():
-            _native.check(self._lib.cvlbm_fno_adam(p.numel(), _native.ptr(p),
-                                                   _native.ptr(self.grads[k]),
-                                                   _native.ptr(st["m"][k]),
-                                                   _native.ptr(st["v"][k]), lr_t, b1, b2, eps,
-                                                   self._s()), "cvlbm_fno_adam")
+        rows = [(p, self.grads[k], st["m"][k], st["v"][k]) for k, p in self.params.items()]
+        n = len(rows)
+        ptrs = [(C.c_void_p * n)(*[r[i].data_ptr() for r in rows]) for i in range(4)]
+        size = (C.c_int64 * n)(*[r[0].numel() for r in rows])
+        _native.check(self._lib.cvlbm_fno_adam_list(n, size, *ptrs, lr_t, b1, b2, eps, self._s()),
+                      "cvlbm_fno_adam_list")
 
     def gemm_ok(self) -> bool:
         return int(self._err.item()) == 0

@@ -505,6 +505,11 @@ int64_t cvlbm_gemm_bf16_workspace(int32_t M, int32_t N, int32_t K);
 int cvlbm_fno_pointwise_fwd(int32_t B, int32_t G, int32_t Cin, int32_t Cout, const float *x,
                             const float *W, const float *bias, const float *s, int32_t act,
                             float *z, float *y, void *stream);
+/* The same with y also stored rounded to bf16 (y_bf16 may be NULL): the operand of
+ * the next spectral transform. */
+int cvlbm_fno_layer_fwd(int32_t B, int32_t G, int32_t Cin, int32_t Cout, const float *x,
+                        const float *W, const float *bias, const float *s, int32_t act, float *z,
+                        float *y, void *y_bf16, void *stream);
 /* dz = dy * gelu'(z) over n elements. */
 int cvlbm_fno_gelu_bwd(int64_t n, const float *z, const float *dy, float *dz, void *stream);
 /* dx (+)= W^T dz (dx may be NULL); dW = sum dz x^T, db = sum dz over samples and
@@ -512,6 +517,12 @@ int cvlbm_fno_gelu_bwd(int64_t n, const float *z, const float *dy, float *dz, vo
 int cvlbm_fno_pointwise_bwd(int32_t B, int32_t G, int32_t Cin, int32_t Cout, const float *dz,
                             const float *x, const float *W, float *dx, int32_t accumulate_dx,
                             float *dW, float *db, float *scratch, void *stream);
+/* One layer's backward pass without dz in memory: dz = dy gelu'(z) (z NULL: dz = dy),
+ * dx = W^T dz (dx may be NULL), dz_bf16 = dz rounded to bf16 (may be NULL), dW and db
+ * as above. */
+int cvlbm_fno_layer_bwd(int32_t B, int32_t G, int32_t Cin, int32_t Cout, const float *dy,
+                        const float *z, const float *x, const float *W, float *dx, void *dz_bf16,
+                        float *dW, float *db, float *scratch, void *stream);
 int64_t cvlbm_fno_pointwise_scratch(int32_t B, int32_t G, int32_t Cin, int32_t Cout);
 /* bh[b][o][k] = sum_i a[b][i][k] R[k][i][o], stored as bf16. */
 int cvlbm_fno_spec_mix_fwd(int32_t B, int32_t C, int32_t M, const float *a, const float *R,
@@ -524,6 +535,16 @@ int cvlbm_fno_to_bf16(int64_t n, const float *src, void *dst, void *stream);
 int cvlbm_fno_mse(int32_t B, int32_t C, int32_t G, const float *y, const float *t,
                   const float *mask, const float *w, float inv_count, float *dy, float *part,
                   int32_t n_parts, void *stream);
+/* cvlbm_fno_mse with inv_count = 1 / max(C * mask_sum[0], 1) formed on the device
+ * (mask_sum: device, the sum of the mask). */
+int cvlbm_fno_mse_mean(int32_t B, int32_t C, int32_t G, const float *y, const float *t,
+                       const float *mask, const float *w, const float *mask_sum, float *dy,
+                       float *part, int32_t n_parts, void *stream);
+/* Adam over `count` tensors (host tables of device pointers and lengths), one launch
+ * per 32 tensors; per element the operations of cvlbm_fno_adam. */
+int cvlbm_fno_adam_list(int32_t count, const int64_t *n, float *const *p, const float *const *g,
+                        float *const *m, float *const *v, float lr, float b1, float b2, float eps,
+                        void *stream);
 /* Adam step, bias correction folded into lr. */
 int cvlbm_fno_adam(int64_t n, float *p, const float *g, float *m, float *v, float lr, float b1,
                    float b2, float eps, void *stream);
