@@ -263,34 +263,48 @@ __global__ void __launch_bounds__(kChunkG)
 // dW[t] (t < n_w) and db[t - n_w] = sum_c part[c][t] in chunk order.
 //
 // One block per 32 sums.  The chain of additions is serial by definition (chunk
-// order), the loads are not: seven warps bring the next 64 partials (rows of 128
-// bytes) into shared memory while warp 0 adds the current 64.  2,048 partials of
-// 1,056 sums: 132 us with one thread per sum loading for itself.
-constexpr int kSumTile = 64;
-__global__ void __launch_bounds__(256)
+// order), the loads are not: eight warps bring the next 128 partials (rows of 128
+// bytes, 16 loads in flight per thread) into shared memory while warp 0 adds the
+// current 128.  2,048 partials of 1,056 sums: 132 us with one thread per sum
+// loading for itself, 75 us with the loads not unrolled.
+constexpr int kSumTile = 128, kSumLoaders = 8;
+__global__ void __launch_bounds__(32 * (kSumLoaders + 1))
     k_sum_parts(int n_parts, int width, int n_w, const float* __restrict__ part,
                 float* __restrict__ dW, float* __restrict__ db) {
   __shared__ float tile[2][kSumTile][32];
-  const int t0 = blockIdx.x * 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int t = t0 + lane;
-  auto fill = [&](int s, int c0, int w, int nw) {
-    for (int r = w; r < kSumTile; r += nw)
-      tile[s][r][lane] = (c0 + r < n_parts && t < width) ? part[(size_t)(c0 + r) * width + t] : 0.0f;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t = blockIdx.x * 32 + lane;
+  constexpr int kRows = kSumTile / kSumLoaders;
+  float v[kRows];
+  auto load = [&](int c0) {
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const int c = c0 + (warp - 1) * kRows + r;
+      v[r] = (c < n_parts && t < width) ? part[(size_t)c * width + t] : 0.0f;
+    }
   };
-  fill(0, 0, warp, 8);
+  auto store = [&](int s) {
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) tile[s][(warp - 1) * kRows + r][lane] = v[r];
+  };
+  if (warp > 0) {
+    load(0);
+    store(0);
+  }
   float acc = 0.0f;
   for (int c0 = 0, s = 0; c0 < n_parts; c0 += kSumTile, s ^= 1) {
     __syncthreads();
     if (warp == 0) {
       const int m = n_parts - c0 < kSumTile ? n_parts - c0 : kSumTile;
       if (m == kSumTile) {
-#pragma unroll
+#pragma unroll 32
         for (int r = 0; r < kSumTile; ++r) acc += tile[s][r][lane];
       } else {
         for (int r = 0; r < m; ++r) acc += tile[s][r][lane];
       }
     } else if (c0 + kSumTile < n_parts) {
-      fill(s ^ 1, c0 + kSumTile, warp - 1, 7);
+      load(c0 + kSumTile);
+      store(s ^ 1);
     }
   }
   if (warp == 0 && t < width) {
@@ -570,7 +584,7 @@ int pointwise_bwd(int32_t B, int32_t G, int32_t Cin, int32_t Cout, const float* 
                                                               dx, d16, scratch, -0.0f);
   cv::count_launches(1);
   const int n_w = Cout * Cin, width = n_w + Cout;
-  k_sum_parts<<<nblk(width, 32), 256, 0, st>>>(nparts, width, n_w, scratch, dW, db);
+  k_sum_parts<<<nblk(width, 32), 32 * (kSumLoaders + 1), 0, st>>>(nparts, width, n_w, scratch, dW, db);
   cv::count_launches(1);
   return check_launch("cvlbm_fno_pointwise_bwd");
 }

@@ -246,11 +246,18 @@ __global__ void __launch_bounds__(128)
 // 128-byte swizzle), so every 64-wide K slice of a 128-row tile is one
 // cp.async.bulk.tensor that lands in the canonical SWIZZLE_128B K-major
 // layout of the tensor core (rows of 128 bytes, 8-row atoms of 1024 bytes,
-// 16-byte chunks permuted by row).  Three stages: one thread issues the TMA
-// loads of slice k + 2 while another has the MMAs of slice k in flight;
-// stage s is refilled once the MMAs that read it have committed to empty[s].
-constexpr int kStagesT = 3;
-
+// 16-byte chunks permuted by row).  ST stages: one thread issues the TMA loads
+// of later slices while another has the MMAs of slice k in flight; stage s is
+// refilled once the MMAs that read it have committed to empty[s].
+//
+// Tile width BN and stages ST (launch rule in launch_tma):
+//  * BN = 128, ST = 3 (97 KB): two CTAs per SM.
+//  * BN = 128, ST = 2 (65 KB): three CTAs per SM, taken when the grid then fits one
+//    wave (the forward transform of the 32 x 32 x 64 lattice: 384 CTAs).
+//  * Few CTAs (a K that does not split): narrower tiles, BN = 64 or 32, with eight
+//    stages, so that more SMs stream the operands; every output element still sums
+//    its K range in the same order.
+//
 // Shared-memory descriptor of a SWIZZLE_128B K-major tile: start address,
 // stride between 8-row atoms 1024 bytes, leading offset unused (1), version
 // 1, layout type 2 (128-byte swizzle).  The K step of 16 elements advances
@@ -289,14 +296,14 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
 // k_gemm_bf16).  Thread 0 issues the TMA loads, thread 32 the MMAs; every
 // wait is bounded, and a CTA that gives up raises the error word, waits
 // (bounded) for the copies and MMAs it started, frees its TMEM and returns.
-template <int BN>
+template <int BN, int ST>
 __global__ void __launch_bounds__(128)
     k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                float* __restrict__ C, float* __restrict__ partial, int M, int N, int kchunk,
                int ldc, int accumulate, int* __restrict__ error) {
   extern __shared__ uint8_t smem_t[];
   constexpr uint32_t kATile = kBM * kBK * 2, kBTile = BN * kBK * 2;
-  __shared__ __align__(8) uint64_t full[kStagesT], empty[kStagesT], done;
+  __shared__ __align__(8) uint64_t full[ST], empty[ST], done;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_fail, s_issued, s_consumed;
   const uint32_t base = (smem_u32(smem_t) + 1023u) & ~1023u;
@@ -311,7 +318,7 @@ __global__ void __launch_bounds__(128)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
   }
   if (tid == 32) {
-    for (int s = 0; s < kStagesT; ++s) {
+    for (int s = 0; s < ST; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&full[s])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&empty[s])));
     }
@@ -327,11 +334,17 @@ __global__ void __launch_bounds__(128)
   const uint32_t tmem = tmem_slot;
   const uint32_t idesc = instr_desc_bf16(kBM, BN);
 
+  if (accumulate && !partial && warp > 1) {
+    // the old values of the tile, on their way to L2 while the MMAs run
+    for (int i = (warp - 2) * 32 + lane; i < kBM * (BN / 32); i += 64)
+      asm volatile("prefetch.global.L2 [%0];\n" ::"l"(C + (size_t)(m0 + i / (BN / 32)) * ldc + n0 +
+                                                     32 * (i % (BN / 32))));
+  }
   if (tid == 0) {
     int kb = 0;
     for (; kb < nk; ++kb) {
-      const int s = kb % kStagesT, j = kb / kStagesT;
-      if (kb >= kStagesT && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((j - 1) & 1))) {
+      const int s = kb % ST, j = kb / ST;
+      if (kb >= ST && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((j - 1) & 1))) {
         s_fail = 1;
         break;
       }
@@ -344,7 +357,7 @@ __global__ void __launch_bounds__(128)
   } else if (tid == 32) {
     int kb = 0;
     for (; kb < nk; ++kb) {
-      const int s = kb % kStagesT, j = kb / kStagesT;
+      const int s = kb % ST, j = kb / ST;
       if (!mbar_wait(smem_u32(&full[s]), (uint32_t)(j & 1))) {
         s_fail = 1;
         break;
@@ -375,37 +388,65 @@ __global__ void __launch_bounds__(128)
       atomicExch(error, 1);
       // loads issued but not consumed still target this CTA's shared memory
       for (int kb = s_consumed; kb < s_issued; ++kb)
-        mbar_wait(smem_u32(&full[kb % kStagesT]), (uint32_t)((kb / kStagesT) & 1));
+        mbar_wait(smem_u32(&full[kb % ST]), (uint32_t)((kb / ST) & 1));
     }
   } else {
-    const int row = m0 + warp * 32 + lane;
-    float* dst = partial ? partial + (size_t)blockIdx.z * M * N + (size_t)row * N + n0
-                         : C + (size_t)row * ldc + n0;
+    // Accumulator rows leave through shared memory (the stages are free now), CW
+    // columns at a time, so that a warp stores whole runs of 4 CW bytes per row.
+    // A lane storing 16 bytes of its own row touched 32 lines per instruction,
+    // and with `accumulate` waited for each such load before the next: 150 us
+    // against 40 us at 128 x 65536 x 768.
+    constexpr int CW = BN < 64 ? BN : 64, LD = CW + 4, LPR = CW / 4, RPI = 32 / LPR, IT = 32 / RPI;
+    float* st = reinterpret_cast<float*>(smem_t + (base - smem_u32(smem_t))) + warp * 32 * LD;
+    const int row0 = m0 + warp * 32;
+    float* dst0 = partial ? partial + (size_t)blockIdx.z * M * N + (size_t)row0 * N + n0
+                          : C + (size_t)row0 * ldc + n0;
+    const size_t ld = partial ? (size_t)N : (size_t)ldc;
     const bool acc = partial == nullptr && accumulate;
-    // 16-byte stores when the row start allows them (partials always do)
-    const bool vec = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+    const bool vec = ((reinterpret_cast<uintptr_t>(dst0) | (ld * sizeof(float))) & 15) == 0;
+    const int r = lane / LPR, cl = 4 * (lane % LPR);
+#pragma unroll 1
+    for (int c0 = 0; c0 < BN; c0 += CW) {
 #pragma unroll
-    for (int c0 = 0; c0 < BN; c0 += 16) {
-      float v[16];
-      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+      for (int cc = 0; cc < CW; cc += 16) {
+        float v[16];
+        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c0 + cc), v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<float4*>(st + lane * LD + cc + 4 * i) =
+              make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+      }
+      __syncwarp();
+      float* d = dst0 + (size_t)r * ld + c0 + cl;
       if (vec) {
-        float4* d4 = reinterpret_cast<float4*>(dst + c0);
+        float4 old[IT];
+        if (acc) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float4 o = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          for (int it = 0; it < IT; ++it)
+            old[it] = *reinterpret_cast<const float4*>(d + (size_t)(it * RPI) * ld);
+        }
+#pragma unroll
+        for (int it = 0; it < IT; ++it) {
+          float4 o = *reinterpret_cast<const float4*>(st + (it * RPI + r) * LD + cl);
           if (acc) {
-            const float4 c = d4[i];
-            o.x = c.x + o.x;
-            o.y = c.y + o.y;
-            o.z = c.z + o.z;
-            o.w = c.w + o.w;
+            o.x = old[it].x + o.x;
+            o.y = old[it].y + o.y;
+            o.z = old[it].z + o.z;
+            o.w = old[it].w + o.w;
           }
-          d4[i] = o;
+          *reinterpret_cast<float4*>(d + (size_t)(it * RPI) * ld) = o;
         }
       } else {
+        for (int it = 0; it < IT; ++it) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) dst[c0 + i] = acc ? dst[c0 + i] + v[i] : v[i];
+          for (int i = 0; i < 4; ++i) {
+            float* e = d + (size_t)(it * RPI) * ld + i;
+            const float o = st[(it * RPI + r) * LD + cl + i];
+            *e = acc ? *e + o : o;
+          }
+        }
       }
+      __syncwarp();
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -455,6 +496,22 @@ bool operand_map(CUtensorMap* map, const void* ptr, int rows, int K, int ld, int
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <int BN, int ST>
+void launch_tma_as(dim3 grid, cudaStream_t s, const CUtensorMap& a, const CUtensorMap& b, float* C,
+                   float* part, int M, int N, int kchunk, int ldc, int accumulate, int* error) {
+  constexpr int smem = ST * (kBM + BN) * kBK * 2 + 1024;
+  static_assert(smem - 1024 >= kBM * ((BN < 64 ? BN : 64) + 4) * 4, "epilogue staging");
+  cudaFuncSetAttribute(k_gemm_tma<BN, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  k_gemm_tma<BN, ST><<<grid, 128, smem, s>>>(a, b, C, part, M, N, kchunk, ldc, accumulate, error);
+}
+
+int sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms > 0 ? sms : 148;
+}
+
 // CVLBM_GEMM_LOADER=threads selects the thread-loaded kernel (comparison).
 bool tma_allowed() {
   const char* e = std::getenv("CVLBM_GEMM_LOADER");
@@ -492,21 +549,25 @@ extern "C" int cvlbm_gemm_bf16(const void* A, const void* B, float* C, int32_t M
   float* part = splits > 1 ? static_cast<float*>(workspace) : nullptr;
   dim3 grid(M / kBM, N / bn, splits);
   const int kchunk = K / splits;
+  // tile width of the TMA form: narrower while most SMs would be idle
+  int bt = bn;
+  const int sms = sm_count();
+  while (bt > 32 && (long long)(M / kBM) * (N / bt) * splits < sms) bt /= 2;
+  const dim3 gt(M / kBM, N / bt, splits);
+  const long long ctas = (long long)gt.x * gt.y * gt.z;
   CUtensorMap mapA, mapB;
   if (tma_allowed() && operand_map(&mapA, A, M, K, lda, kBM) &&
-      operand_map(&mapB, B, N, K, ldb, bn)) {
-    const size_t smem = (size_t)kStagesT * (kBM + bn) * kBK * 2 + 1024;
-    if (bn == 128) {
-      cudaFuncSetAttribute(k_gemm_tma<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
-      k_gemm_tma<128><<<grid, 128, smem, s>>>(mapA, mapB, C, part, M, N, kchunk, ldc, accumulate,
-                                              error);
-    } else {
-      cudaFuncSetAttribute(k_gemm_tma<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
-      k_gemm_tma<64><<<grid, 128, smem, s>>>(mapA, mapB, C, part, M, N, kchunk, ldc, accumulate,
-                                             error);
-    }
+      operand_map(&mapB, B, N, K, ldb, bt)) {
+    if (bt == 128 && ctas > 2LL * sms && ctas <= 3LL * sms)
+      launch_tma_as<128, 2>(gt, s, mapA, mapB, C, part, M, N, kchunk, ldc, accumulate, error);
+    else if (bt == 128)
+      launch_tma_as<128, 3>(gt, s, mapA, mapB, C, part, M, N, kchunk, ldc, accumulate, error);
+    else if (bt == 64 && ctas > sms)
+      launch_tma_as<64, 3>(gt, s, mapA, mapB, C, part, M, N, kchunk, ldc, accumulate, error);
+    else if (bt == 64)
+      launch_tma_as<64, 8>(gt, s, mapA, mapB, C, part, M, N, kchunk, ldc, accumulate, error);
+    else
+      launch_tma_as<32, 8>(gt, s, mapA, mapB, C, part, M, N, kchunk, ldc, accumulate, error);
   } else if (bn == 128) {
     const size_t smem = 2 * (kBM + 128) * kBK * 2;
     cudaFuncSetAttribute(k_gemm_bf16<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
