@@ -113,15 +113,24 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
   for (int i = 0; i < CI; ++i)
     xi[i] = i < Cin ? ld_pair(x + ((size_t)b * Cin + i) * G, g, G, vec) : make_float2(0.0f, 0.0f);
+  // s of four outputs, loaded one group ahead of its use
+  auto load_s = [&](int o, float2* v) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      v[k] = (s && o + k < Cout) ? ld_pair(s + ((size_t)b * Cout + o + k) * G, g, G, vec)
+                                 : make_float2(0.0f, 0.0f);
+  };
+  float2 sv[4], sn[4];
+  load_s(0, sn);
 #pragma unroll 1
   for (int o = 0; o < Cout; o += 4) {
-    float2 acc[4], sv[4];
+    float2 acc[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       acc[k] = make_float2(sb[o + k], sb[o + k]);
-      sv[k] = (s && o + k < Cout) ? ld_pair(s + ((size_t)b * Cout + o + k) * G, g, G, vec)
-                                  : make_float2(0.0f, 0.0f);
+      sv[k] = sn[k];
     }
+    load_s(o + 4, sn);
 #pragma unroll
     for (int i = 0; i < CI; ++i) {
       const float4 w0 = sW[i][o / 2], w1 = sW[i][o / 2 + 1];
@@ -162,7 +171,7 @@ __global__ void k_gelu_bwd(long long n, const float* __restrict__ z, const float
 // eight lanes fall into distinct banks), packed fp32 over the output pairs.
 constexpr int kChunkG = 128;
 template <int CI, int CO>
-__global__ void __launch_bounds__(kChunkG)
+__global__ void __launch_bounds__(kChunkG, 5)
     k_pointwise_bwd(int B, int G, int Cin, int Cout, const float* __restrict__ dy,
                     const float* __restrict__ z, const float* __restrict__ x,
                     const float* __restrict__ W, int accumulate, float* __restrict__ dx,
@@ -178,31 +187,45 @@ __global__ void __launch_bounds__(kChunkG)
   const int chunks = (G + kChunkG - 1) / kChunkG;
   const int c = blockIdx.x, b = c / chunks, g = (c % chunks) * kChunkG + tid;
   const bool ok = g < G;
+  // x goes to shared memory by itself (4-byte asynchronous copies) while dz forms
+#pragma unroll
+  for (int i = 0; i < CI; ++i) {
+    const bool in = ok && i < Cin;
+    const float* src = x + ((size_t)b * Cin + (in ? i : 0)) * G + (ok ? g : 0);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(&sx[tid][i]))),
+                 "l"(src), "r"(in ? 4 : 0)
+                 : "memory");
+  }
   float d[CO];
+  constexpr int kOC = CO < 16 ? CO : 16;  // channels whose dy and z are in flight together
 #pragma unroll
-  for (int o = 0; o < CO; ++o)
-    d[o] = (ok && o < Cout) ? dy[((size_t)b * Cout + o) * G + g] : 0.0f;
-  if (z) {
+  for (int o0 = 0; o0 < CO; o0 += kOC) {
+    float zv[kOC];
 #pragma unroll
-    for (int o = 0; o < CO; ++o)
-      if (ok && o < Cout) d[o] = d[o] * gelu_grad(z[((size_t)b * Cout + o) * G + g]);
+    for (int k = 0; k < kOC; ++k) {
+      const int o = o0 + k;
+      const size_t at = ((size_t)b * Cout + o) * G + g;
+      d[o] = (ok && o < Cout) ? dy[at] : 0.0f;
+      zv[k] = (z && ok && o < Cout) ? z[at] : 0.0f;
+    }
+    if (z) {
+#pragma unroll
+      for (int k = 0; k < kOC; ++k) d[o0 + k] = d[o0 + k] * gelu_grad(zv[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kOC; k += 4)
+      *reinterpret_cast<float4*>(&sdz[tid][o0 + k]) =
+          make_float4(d[o0 + k], d[o0 + k + 1], d[o0 + k + 2], d[o0 + k + 3]);
+    if (dzb) {
+#pragma unroll
+      for (int k = 0; k < kOC; ++k) {
+        const int o = o0 + k;
+        if (ok && o < Cout) dzb[((size_t)b * Cout + o) * G + g] = __float2bfloat16_rn(d[o]);
+      }
+    }
   }
-  if (dzb) {
-#pragma unroll
-    for (int o = 0; o < CO; ++o)
-      if (ok && o < Cout) dzb[((size_t)b * Cout + o) * G + g] = __float2bfloat16_rn(d[o]);
-  }
-#pragma unroll
-  for (int o = 0; o < CO; o += 4)
-    *reinterpret_cast<float4*>(&sdz[tid][o]) = make_float4(d[o], d[o + 1], d[o + 2], d[o + 3]);
-#pragma unroll
-  for (int i = 0; i < CI; i += 4) {
-    float v[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      v[k] = (ok && i + k < Cin) ? x[((size_t)b * Cin + i + k) * G + g] : 0.0f;
-    *reinterpret_cast<float4*>(&sx[tid][i]) = make_float4(v[0], v[1], v[2], v[3]);
-  }
+  asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
   if (dx && ok) {
 #pragma unroll 1
@@ -263,15 +286,15 @@ __global__ void __launch_bounds__(kChunkG)
 // dW[t] (t < n_w) and db[t - n_w] = sum_c part[c][t] in chunk order.
 //
 // One block per 32 sums.  The chain of additions is serial by definition (chunk
-// order), the loads are not: eight warps bring the next 128 partials (rows of 128
-// bytes, 16 loads in flight per thread) into shared memory while warp 0 adds the
-// current 128.  2,048 partials of 1,056 sums: 132 us with one thread per sum
-// loading for itself, 75 us with the loads not unrolled.
-constexpr int kSumTile = 128, kSumLoaders = 8;
+// order), the loads are not: eight warps bring the next 256 partials (rows of 128
+// bytes, 32 loads in flight per thread) while warp 0 adds the current 256 from
+// shared memory.  2,048 partials of 1,056 sums: 132 us with one thread per sum
+// loading for itself, 75 us with the loads not unrolled, 27 us with 16 in flight.
+constexpr int kSumTile = 256, kSumLoaders = 8;
 __global__ void __launch_bounds__(32 * (kSumLoaders + 1))
     k_sum_parts(int n_parts, int width, int n_w, const float* __restrict__ part,
                 float* __restrict__ dW, float* __restrict__ db) {
-  __shared__ float tile[2][kSumTile][32];
+  __shared__ float tile[kSumTile][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = blockIdx.x * 32 + lane;
   constexpr int kRows = kSumTile / kSumLoaders;
@@ -283,29 +306,26 @@ __global__ void __launch_bounds__(32 * (kSumLoaders + 1))
       v[r] = (c < n_parts && t < width) ? part[(size_t)c * width + t] : 0.0f;
     }
   };
-  auto store = [&](int s) {
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) tile[s][(warp - 1) * kRows + r][lane] = v[r];
-  };
-  if (warp > 0) {
-    load(0);
-    store(0);
-  }
+  if (warp > 0) load(0);
   float acc = 0.0f;
-  for (int c0 = 0, s = 0; c0 < n_parts; c0 += kSumTile, s ^= 1) {
+  for (int c0 = 0; c0 < n_parts; c0 += kSumTile) {
+    if (warp > 0) {
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) tile[(warp - 1) * kRows + r][lane] = v[r];
+    }
     __syncthreads();
     if (warp == 0) {
       const int m = n_parts - c0 < kSumTile ? n_parts - c0 : kSumTile;
       if (m == kSumTile) {
 #pragma unroll 32
-        for (int r = 0; r < kSumTile; ++r) acc += tile[s][r][lane];
+        for (int r = 0; r < kSumTile; ++r) acc += tile[r][lane];
       } else {
-        for (int r = 0; r < m; ++r) acc += tile[s][r][lane];
+        for (int r = 0; r < m; ++r) acc += tile[r][lane];
       }
     } else if (c0 + kSumTile < n_parts) {
       load(c0 + kSumTile);
-      store(s ^ 1);
     }
+    __syncthreads();
   }
   if (warp == 0 && t < width) {
     if (t < n_w)
@@ -320,10 +340,10 @@ __global__ void __launch_bounds__(32 * (kSumLoaders + 1))
 //
 // Bound by the weights (R: 3.1 MB at 768 modes, read once) and by latency: a warp
 // owns one mode with lane = output channel, so R[k] is read in 128-byte rows; the
-// block's eight modes of a (32-byte runs) are staged in shared memory and the
+// block's four modes of a (16-byte runs) are staged in shared memory and the
 // results leave through it.  One thread per (sample, mode), each walking its own
 // 4 KB of R, took 100 us.
-constexpr int kMixK = 8, kMixB = 4;  // modes per block, samples per pass
+constexpr int kMixK = 4, kMixB = 4;  // modes per block, samples per pass
 __global__ void __launch_bounds__(32 * kMixK)
     k_spec_mix_fwd(int B, int C, int M, const float* __restrict__ a, const float* __restrict__ R,
                    __nv_bfloat16* __restrict__ bh) {
@@ -337,9 +357,16 @@ __global__ void __launch_bounds__(32 * kMixK)
     r[i] = (k < M && i < C && lane < C) ? Rk[i * C + lane] : 0.0f;
   for (int b0 = 0; b0 < B; b0 += kMixB) {
     const int rows = (B - b0 < kMixB ? B - b0 : kMixB) * C;
-    for (int t = threadIdx.x; t < rows * kMixK; t += blockDim.x) {
-      const int row = t / kMixK, kk = t % kMixK;
-      sa[row][kk] = k0 + kk < M ? a[((size_t)b0 * C + row) * M + k0 + kk] : 0.0f;
+    float ta[kMixB];
+#pragma unroll
+    for (int u = 0; u < kMixB; ++u) {
+      const int t = threadIdx.x + u * 32 * kMixK, row = t / kMixK, kk = t % kMixK;
+      ta[u] = (row < rows && k0 + kk < M) ? a[((size_t)b0 * C + row) * M + k0 + kk] : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kMixB; ++u) {
+      const int t = threadIdx.x + u * 32 * kMixK, row = t / kMixK, kk = t % kMixK;
+      sa[row][kk] = ta[u];
     }
     __syncthreads();
     float acc[kMixB];
@@ -385,19 +412,29 @@ __global__ void __launch_bounds__(32 * kMixK)
   const bool live = k < M && lane < C;
   float* Rw = sR + w * kMaxC * (kMaxC + 1);
   const float* Rk = R + (size_t)k * C * C;
+  float dr[kMaxC];  // R[k] on its way to shared memory (all loads in flight), then dR[k]
 #pragma unroll
-  for (int i = 0; i < kMaxC; ++i)
-    if (i < C) Rw[i * (kMaxC + 1) + lane] = live ? Rk[i * C + lane] : 0.0f;
-  float dr[kMaxC];
+  for (int i = 0; i < kMaxC; ++i) dr[i] = (live && i < C) ? Rk[i * C + lane] : 0.0f;
+#pragma unroll
+  for (int i = 0; i < kMaxC; ++i) Rw[i * (kMaxC + 1) + lane] = dr[i];
 #pragma unroll
   for (int i = 0; i < kMaxC; ++i) dr[i] = 0.0f;
   for (int b0 = 0; b0 < B; b0 += kMixB) {
     const int rows = (B - b0 < kMixB ? B - b0 : kMixB) * C;
-    for (int t = threadIdx.x; t < rows * kMixK; t += blockDim.x) {
-      const int row = t / kMixK, kk = t % kMixK;
-      const size_t at = ((size_t)b0 * C + row) * M + k0 + kk;
-      sa[row * (kMixK + 1) + kk] = k0 + kk < M ? a[at] : 0.0f;
-      sd[row * (kMixK + 1) + kk] = k0 + kk < M ? dbh[at] : 0.0f;
+    float ta[kMixB], td[kMixB];
+#pragma unroll
+    for (int u = 0; u < kMixB; ++u) {
+      const int t = threadIdx.x + u * 32 * kMixK, row = t / kMixK, kk = t % kMixK;
+      const bool in = row < rows && k0 + kk < M;
+      const size_t at = in ? ((size_t)b0 * C + row) * M + k0 + kk : 0;
+      ta[u] = in ? a[at] : 0.0f;
+      td[u] = in ? dbh[at] : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kMixB; ++u) {
+      const int t = threadIdx.x + u * 32 * kMixK, row = t / kMixK, kk = t % kMixK;
+      sa[row * (kMixK + 1) + kk] = ta[u];
+      sd[row * (kMixK + 1) + kk] = td[u];
     }
     __syncthreads();
     if (live) {

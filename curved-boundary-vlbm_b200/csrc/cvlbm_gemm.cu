@@ -254,9 +254,11 @@ __global__ void __launch_bounds__(128)
 //  * BN = 128, ST = 3 (97 KB): two CTAs per SM.
 //  * BN = 128, ST = 2 (65 KB): three CTAs per SM, taken when the grid then fits one
 //    wave (the forward transform of the 32 x 32 x 64 lattice: 384 CTAs).
-//  * Few CTAs (a K that does not split): narrower tiles, BN = 64 or 32, with eight
-//    stages, so that more SMs stream the operands; every output element still sums
-//    its K range in the same order.
+//  * Few CTAs (a K that does not split): BN = 64 with six stages.  The CTA is then
+//    bound by its chain of dependent MMAs (one 16-deep step of K after the other
+//    into the same accumulators, about 78 ns each at N = 64 or 32, 100 ns at 128):
+//    128 x 768 x 93312 in two splits 228 us against 291; narrower tiles and more
+//    stages measured the same.  Every element sums its K range in the same order.
 //
 // Shared-memory descriptor of a SWIZZLE_128B K-major tile: start address,
 // stride between 8-row atoms 1024 bytes, leading offset unused (1), version
@@ -552,7 +554,7 @@ extern "C" int cvlbm_gemm_bf16(const void* A, const void* B, float* C, int32_t M
   // tile width of the TMA form: narrower while most SMs would be idle
   int bt = bn;
   const int sms = sm_count();
-  while (bt > 32 && (long long)(M / kBM) * (N / bt) * splits < sms) bt /= 2;
+  while (bt > 64 && (long long)(M / kBM) * (N / bt) * splits < sms) bt /= 2;
   const dim3 gt(M / kBM, N / bt, splits);
   const long long ctas = (long long)gt.x * gt.y * gt.z;
   CUtensorMap mapA, mapB;
@@ -564,10 +566,8 @@ extern "C" int cvlbm_gemm_bf16(const void* A, const void* B, float* C, int32_t M
       launch_tma_as<128, 3>(gt, s, mapA, mapB, C, part, M, N, kchunk, ldc, accumulate, error);
     else if (bt == 64 && ctas > sms)
       launch_tma_as<64, 3>(gt, s, mapA, mapB, C, part, M, N, kchunk, ldc, accumulate, error);
-    else if (bt == 64)
-      launch_tma_as<64, 8>(gt, s, mapA, mapB, C, part, M, N, kchunk, ldc, accumulate, error);
     else
-      launch_tma_as<32, 8>(gt, s, mapA, mapB, C, part, M, N, kchunk, ldc, accumulate, error);
+      launch_tma_as<64, 6>(gt, s, mapA, mapB, C, part, M, N, kchunk, ldc, accumulate, error);
   } else if (bn == 128) {
     const size_t smem = 2 * (kBM + 128) * kBK * 2;
     cudaFuncSetAttribute(k_gemm_bf16<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
