@@ -46,12 +46,31 @@ struct Ctx2 {
   double den;   // damping: 1 + 0.5 dt gamma (else 1)
   double dt_om; // dt / omega
   double src_w; // dt (1/omega - 0.5) * 0.25, the source weight of a characteristic row
+  DivC dden;    // division by den
+  DivC dx1, dx2, dy1, dy2;  // divisions by dx, 2 dx, dy, 2 dy
 };
 
 // Boundary time: the step's start time (host value, or the device clock in
 // graph mode) plus `offset`, evaluated as the reference's time + 0.5*dt.
 __device__ __forceinline__ double time_of(const double* clock, double t, double offset) {
   return (clock ? clock[0] : t) + offset;
+}
+
+// Source / damping half step of the moments (two_d/curved_boundary_warp.py:1735-1756).
+__device__ __forceinline__ void source_half2(const Ctx2& c, double* S) {
+  if (c.p.source_mode == kSrcConstant) {
+#pragma unroll
+    for (int a = 0; a < kC2; ++a) S[a] += c.hdt * c.p.source[a];
+  } else if (c.p.source_mode == kSrcDamping) {
+    S[0] = divc(S[0], c.dden);
+    S[1] = divc(S[1], c.dden);
+  }
+}
+
+// Jacobi quotient of the displacement sweep: an interior node's weight sum is
+// exactly 4, and a product with 1/4 rounds as the division does.
+__device__ __forceinline__ double sweep_quot2(double r, double diag) {
+  return diag == 4.0 ? r * 0.25 : r / diag;
 }
 
 // ---------------------------------------------------------------------------
@@ -84,15 +103,7 @@ __global__ void __launch_bounds__(256) k_collide2(Ctx2 c, const double* __restri
     for (int q = 0; q < kQ2; ++q) s += f[q * kC2 + a];
     S[a] = s;
   }
-  const double hdt = 0.5 * p.dt;
-  if (p.source_mode == kSrcConstant) {
-#pragma unroll
-    for (int a = 0; a < kC2; ++a) S[a] += hdt * p.source[a];
-  } else if (p.source_mode == kSrcDamping) {
-    double den = 1.0 + hdt * p.source[0];
-    S[0] = S[0] / den;
-    S[1] = S[1] / den;
-  }
+  source_half2(c, S);
   double B[kC2];
 #pragma unroll
   for (int a = 0; a < kC2; ++a) B[a] = source_comp(a, p.source_mode, p.source, S);
@@ -155,15 +166,7 @@ __global__ void __launch_bounds__(256) k_collide2_mrt(Ctx2 c, const double* __re
     for (int q = 0; q < kQ2; ++q) s += f[q * kC2 + a];
     S[a] = s;
   }
-  const double hdt = 0.5 * p.dt;
-  if (p.source_mode == kSrcConstant) {
-#pragma unroll
-    for (int a = 0; a < kC2; ++a) S[a] += hdt * p.source[a];
-  } else if (p.source_mode == kSrcDamping) {
-    double den = 1.0 + hdt * p.source[0];
-    S[0] = S[0] / den;
-    S[1] = S[1] / den;
-  }
+  source_half2(c, S);
 #pragma unroll
   for (int a = 0; a < kC2; ++a) U[(size_t)a * N + n] = S[a];
   double ux = ustar[n] + 0.5 * p.dt * S[0];
@@ -318,8 +321,8 @@ __global__ void __launch_bounds__(256) k_sweep2(Ctx2 c, const double* __restrict
   double u0 = u[n], u1 = u[N + n];
   double n0 = u0, n1 = u1;
   if (diag > 0.0) {
-    n0 = u0 + p.relax * (rx / diag - u0);
-    n1 = u1 + p.relax * (ry / diag - u1);
+    n0 = u0 + p.relax * (sweep_quot2(rx, diag) - u0);
+    n1 = u1 + p.relax * (sweep_quot2(ry, diag) - u1);
   }
   unext[n] = n0;
   unext[N + n] = n1;
@@ -338,20 +341,20 @@ __global__ void k_commit2(int N2, const double* __restrict__ src, double* __rest
 // (_local_dudx/_local_dudy) and :3521-3615.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double dudx2(const double* uc, const int* act, int n, int i, int nx,
-                                        int stride, double h) {
+                                        int stride, const DivC& h1, const DivC& h2) {
   // stride = ny for d/dx, 1 for d/dy; i is the index along that axis
   bool am = i > 0 && act[n - stride] != 0;
   bool ap = i + 1 < nx && act[n + stride] != 0;
-  if (am && ap) return (uc[n + stride] - uc[n - stride]) / (2.0 * h);
+  if (am && ap) return divc(uc[n + stride] - uc[n - stride], h2);
   if (ap) {
     if (i + 2 < nx && act[n + 2 * stride] != 0)
-      return (-3.0 * uc[n] + 4.0 * uc[n + stride] - uc[n + 2 * stride]) / (2.0 * h);
-    return (uc[n + stride] - uc[n]) / h;
+      return divc(-3.0 * uc[n] + 4.0 * uc[n + stride] - uc[n + 2 * stride], h2);
+    return divc(uc[n + stride] - uc[n], h1);
   }
   if (am) {
     if (i > 1 && act[n - 2 * stride] != 0)
-      return (3.0 * uc[n] - 4.0 * uc[n - stride] + uc[n - 2 * stride]) / (2.0 * h);
-    return (uc[n] - uc[n - stride]) / h;
+      return divc(3.0 * uc[n] - 4.0 * uc[n - stride] + uc[n - 2 * stride], h2);
+    return divc(uc[n] - uc[n - stride], h1);
   }
   return 0.0;
 }
@@ -372,10 +375,10 @@ __global__ void __launch_bounds__(256) k_repair2(Ctx2 c, double* __restrict__ f,
     if (act[n - ny] == 0 || act[n + ny] == 0 || act[n - 1] == 0 || act[n + 1] == 0) return;
   }
   double o11 = U[2 * N + n], o12 = U[3 * N + n], o21 = U[4 * N + n], o22 = U[5 * N + n];
-  double t11 = 1.0 + dudx2(u, act, n, i, nx, ny, p.dx);
-  double t12 = dudx2(u, act, n, j, ny, 1, p.dy);
-  double t21 = dudx2(u + N, act, n, i, nx, ny, p.dx);
-  double t22 = 1.0 + dudx2(u + N, act, n, j, ny, 1, p.dy);
+  double t11 = 1.0 + dudx2(u, act, n, i, nx, ny, c.dx1, c.dx2);
+  double t12 = dudx2(u, act, n, j, ny, 1, c.dy1, c.dy2);
+  double t21 = dudx2(u + N, act, n, i, nx, ny, c.dx1, c.dx2);
+  double t22 = 1.0 + dudx2(u + N, act, n, j, ny, 1, c.dy1, c.dy2);
   double alpha = fmax(0.0, fmin(1.0, p.blend));
   double n11 = o11, n12 = o12, n21 = o21, n22 = o22;
   for (int g = 0; g < 10; ++g) {
@@ -498,14 +501,7 @@ __global__ void __launch_bounds__(256) k_refresh2(Ctx2 c, const double* __restri
     for (int q = 0; q < kQ2; ++q) s += f0[(size_t)(q * kC2 + a) * N + n];
     S[a] = s;
   }
-  const double hdt = 0.5 * p.dt;
-  if (p.source_mode == kSrcConstant) {
-    for (int a = 0; a < kC2; ++a) S[a] += hdt * p.source[a];
-  } else if (p.source_mode == kSrcDamping) {
-    double den = 1.0 + hdt * p.source[0];
-    S[0] = S[0] / den;
-    S[1] = S[1] / den;
-  }
+  source_half2(c, S);
   for (int a = 0; a < kC2; ++a) U[(size_t)a * N + n] = S[a];
   u[n] = ustar[n] + 0.5 * p.dt * S[0];
   u[N + n] = ustar[N + n] + 0.5 * p.dt * S[1];
@@ -580,6 +576,11 @@ Ctx2 make_ctx(const cvlbm2d_problem* p) {
   c.ff = 0.5 / p->c;
   c.hdt = 0.5 * p->dt;
   c.den = p->source_mode == kSrcDamping ? 1.0 + c.hdt * p->source[0] : 1.0;
+  c.dden = make_divc(c.den);
+  c.dx1 = make_divc(p->dx);
+  c.dx2 = make_divc(2.0 * p->dx);
+  c.dy1 = make_divc(p->dy);
+  c.dy2 = make_divc(2.0 * p->dy);
   c.dt_om = p->dt / p->omega;
   c.src_w = p->dt * (1.0 / p->omega - 0.5) * 0.25;
   return c;

@@ -36,27 +36,7 @@ struct Fused2 {
 };
 
 // Moments of node n (reference order: for q: for a) with the collision's
-// source / damping half step (two_d/curved_boundary_warp.py:1735-1756).
-__device__ __forceinline__ void moments2(const cvlbm2d_problem& p, const double* __restrict__ f0,
-                                         int N, int n, double* S) {
-#pragma unroll
-  for (int a = 0; a < 6; ++a) S[a] = 0.0;
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int a = 0; a < 6; ++a) S[a] += f0[(size_t)(q * 6 + a) * N + n];
-  const double hdt = 0.5 * p.dt;
-  if (p.source_mode == kSrcConstant) {
-#pragma unroll
-    for (int a = 0; a < 6; ++a) S[a] += hdt * p.source[a];
-  } else if (p.source_mode == kSrcDamping) {
-    double den = 1.0 + hdt * p.source[0];
-    S[0] = S[0] / den;
-    S[1] = S[1] / den;
-  }
-}
-
-// moments2 with the per-problem constants of Ctx2 (the same doubles)
+// source / damping half step.  32-bit offsets: callers hold 24 nx ny < 2^31.
 __device__ __forceinline__ void moments2c(const Ctx2& c, const double* __restrict__ f0, int n,
                                           double* S) {
   const int N = c.N;
@@ -66,13 +46,7 @@ __device__ __forceinline__ void moments2c(const Ctx2& c, const double* __restric
   for (int q = 0; q < 4; ++q)
 #pragma unroll
     for (int a = 0; a < 6; ++a) S[a] += f0[(q * 6 + a) * N + n];
-  if (c.p.source_mode == kSrcConstant) {
-#pragma unroll
-    for (int a = 0; a < 6; ++a) S[a] += c.hdt * c.p.source[a];
-  } else if (c.p.source_mode == kSrcDamping) {
-    S[0] = S[0] / c.den;
-    S[1] = S[1] / c.den;
-  }
+  source_half2(c, S);
 }
 
 // Region flags in shared memory: bit 0 active, bit 1 holds a cut link
@@ -146,13 +120,7 @@ __device__ __forceinline__ void fused2_tile(
           sfo[(q * 6 + a) * kTN + threadIdx.x] = v;
           S[a] += v;
         }
-      if (p.source_mode == kSrcConstant) {
-#pragma unroll
-        for (int a = 0; a < 6; ++a) S[a] += c.hdt * p.source[a];
-      } else if (p.source_mode == kSrcDamping) {
-        S[0] = S[0] / c.den;
-        S[1] = S[1] / c.den;
-      }
+      source_half2(c, S);
       ucol0 = ustar[n] + c.hdt * S[0];
       ucol1 = ustar[N + n] + c.hdt * S[1];
     } else {
@@ -296,8 +264,8 @@ __device__ __forceinline__ void fused2_tile(
     }
     double u0 = sU[0][r], u1 = sU[1][r];
     if (diag > 0.0) {
-      u0 = u0 + p.relax * (rx / diag - u0);
-      u1 = u1 + p.relax * (ry / diag - u1);
+      u0 = u0 + p.relax * (sweep_quot2(rx, diag) - u0);
+      u1 = u1 + p.relax * (sweep_quot2(ry, diag) - u1);
     }
     sN[0][s] = u0;
     sN[1][s] = u1;
@@ -325,24 +293,25 @@ __device__ __forceinline__ void fused2_tile(
       for (int ax = 0; ax < 2; ++ax) {
         const int rs = ax == 0 ? kRX : 1, ss = ax == 0 ? kSX : 1;
         const int ii = ax == 0 ? i : j, nn = ax == 0 ? nx : ny;
-        const double h = ax == 0 ? p.dx : p.dy;
+        const DivC& h1 = ax == 0 ? c.dx1 : c.dy1;
+        const DivC& h2 = ax == 0 ? c.dx2 : c.dy2;
         const bool am = ii > 0 && sA[r_own - rs], ap = ii + 1 < nn && sA[r_own + rs];
 #pragma unroll
         for (int comp = 0; comp < 2; ++comp) {
           const double* w = sN[comp];
           double d;
           if (am && ap) {
-            d = (w[s_own + ss] - w[s_own - ss]) / (2.0 * h);
+            d = divc(w[s_own + ss] - w[s_own - ss], h2);
           } else if (ap) {
             if (ii + 2 < nn && sA[r_own + 2 * rs])
-              d = (-3.0 * w[s_own] + 4.0 * w[s_own + ss] - w[s_own + 2 * ss]) / (2.0 * h);
+              d = divc(-3.0 * w[s_own] + 4.0 * w[s_own + ss] - w[s_own + 2 * ss], h2);
             else
-              d = (w[s_own + ss] - w[s_own]) / h;
+              d = divc(w[s_own + ss] - w[s_own], h1);
           } else if (am) {
             if (ii > 1 && sA[r_own - 2 * rs])
-              d = (3.0 * w[s_own] - 4.0 * w[s_own - ss] + w[s_own - 2 * ss]) / (2.0 * h);
+              d = divc(3.0 * w[s_own] - 4.0 * w[s_own - ss] + w[s_own - 2 * ss], h2);
             else
-              d = (w[s_own] - w[s_own - ss]) / h;
+              d = divc(w[s_own] - w[s_own - ss], h1);
           } else {
             d = 0.0;
           }
@@ -492,7 +461,7 @@ __global__ void __launch_bounds__(kTX * TY)
   const int n = i * p.ny + j;
   if (p.active[n] == 0) return;
   double S[6];
-  moments2(p, f0, N, n, S);
+  moments2c(c, f0, n, S);
 #pragma unroll
   for (int a = 0; a < 6; ++a) mom[(size_t)a * N + n] = S[a];
   mom[6 * (size_t)N + n] = ustar[n] + 0.5 * p.dt * S[0];

@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(256)
   const cvlbm2d_problem& p = c.p;
   if (p.active[n] == 0) return;
   double S[6];
-  moments2(p, f0, N, n, S);
+  moments2c(c, f0, n, S);
 #pragma unroll
   for (int a = 0; a < 6; ++a) U[(size_t)a * N + n] = S[a];
   const double u0 = ustar[n] + 0.5 * p.dt * S[0];
@@ -91,8 +91,8 @@ __global__ void __launch_bounds__(256)
   const double u0 = ucol[n], u1 = ucol[N + n];
   double n0 = u0, n1 = u1;
   if (diag > 0.0) {
-    n0 = u0 + p.relax * (rx / diag - u0);
-    n1 = u1 + p.relax * (ry / diag - u1);
+    n0 = u0 + p.relax * (sweep_quot2(rx, diag) - u0);
+    n1 = u1 + p.relax * (sweep_quot2(ry, diag) - u1);
   }
   u[n] = n0;
   u[N + n] = n1;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(128)
   const int i = n / ny, j = n - i * ny;
   const Mat& m = c.m;
   double S[6];
-  moments2(p, f0, N, n, S);
+  moments2c(c, f0, n, S);
   double Fn[4] = {S[2], S[3], S[4], S[5]};
   bool repaired = false;
   if (do_repair) {
@@ -124,10 +124,10 @@ __global__ void __launch_bounds__(128)
       ok = i > 0 && i + 1 < nx && j > 0 && j + 1 < ny && act[n - ny] && act[n + ny] &&
            act[n - 1] && act[n + 1];
     if (ok) {
-      const double t11 = 1.0 + dudx2(u, act, n, i, nx, ny, p.dx);
-      const double t12 = dudx2(u, act, n, j, ny, 1, p.dy);
-      const double t21 = dudx2(u + N, act, n, i, nx, ny, p.dx);
-      const double t22 = 1.0 + dudx2(u + N, act, n, j, ny, 1, p.dy);
+      const double t11 = 1.0 + dudx2(u, act, n, i, nx, ny, c.dx1, c.dx2);
+      const double t12 = dudx2(u, act, n, j, ny, 1, c.dy1, c.dy2);
+      const double t21 = dudx2(u + N, act, n, i, nx, ny, c.dx1, c.dx2);
+      const double t22 = 1.0 + dudx2(u + N, act, n, j, ny, 1, c.dy1, c.dy2);
       double alpha = fmax(0.0, fmin(1.0, p.blend));
       for (int it = 0; it < 10; ++it) {
         Fn[0] = S[2] + alpha * (t11 - S[2]);

@@ -37,7 +37,30 @@ struct Ctx3 {
   cvlbm3d_problem p;
   Mat m;
   int N;
+  // per-problem constants, formed once on the host with the operations the kernels
+  // would otherwise repeat per node, and the divisions by constants
+  double hdt, k3c, ff, sw;  // dt/2, 3/c, 0.5/c, dt (2 - omega) / 12
+  DivC dden;                // 1 + dt/2 gamma (damping)
+  DivC h1[3], h2[3];        // dx, dy, dz and twice each
+  DivC d6, dc, d3;          // 6, c, 3
 };
+
+// Source / damping half step of the moments.
+__device__ __forceinline__ void source_half3(const Ctx3& c, double* S) {
+  if (c.p.source_mode == kSrcConstant) {
+#pragma unroll
+    for (int a = 0; a < kC3; ++a) S[a] += c.hdt * c.p.source[a];
+  } else if (c.p.source_mode == kSrcDamping) {
+    S[0] = divc(S[0], c.dden);
+    S[1] = divc(S[1], c.dden);
+    S[2] = divc(S[2], c.dden);
+  }
+}
+
+// Jacobi quotient of the displacement sweep (an interior node's weight sum is 6).
+__device__ __forceinline__ double sweep_quot3(const Ctx3& c, double r, double d) {
+  return d == 6.0 ? divc(r, c.d6) : r / d;
+}
 
 __device__ __forceinline__ double time_of(const double* clock, double t, double offset) {
   return (clock ? clock[0] : t) + offset;
@@ -63,15 +86,7 @@ __global__ void __launch_bounds__(128) k_collide3(Ctx3 c, double* __restrict__ f
     S[a] = s;
   }
   const double hdt = 0.5 * p.dt;
-  if (p.source_mode == kSrcConstant) {
-#pragma unroll
-    for (int a = 0; a < kC3; ++a) S[a] += hdt * p.source[a];
-  } else if (p.source_mode == kSrcDamping) {
-    double den = 1.0 + hdt * p.source[0];
-    S[0] = S[0] / den;
-    S[1] = S[1] / den;
-    S[2] = S[2] / den;
-  }
+  source_half3(c, S);
 #pragma unroll
   for (int a = 0; a < kC3; ++a) U[(size_t)a * N + n] = S[a];
 #pragma unroll
@@ -164,7 +179,7 @@ __global__ void __launch_bounds__(256) k_sweep3(Ctx3 c, const double* __restrict
   for (int comp = 0; comp < 3; ++comp) {
     double uo = u[(size_t)comp * N + n];
     double un = uo;
-    if (d[comp] > 0.0) un = uo + p.relax * (r[comp] / d[comp] - uo);
+    if (d[comp] > 0.0) un = uo + p.relax * (sweep_quot3(c, r[comp], d[comp]) - uo);
     unext[(size_t)comp * N + n] = un;
     ustar[(size_t)comp * N + n] = ustar[(size_t)comp * N + n] + (un - uo);
   }
@@ -179,19 +194,19 @@ __global__ void k_copy3(long long n3, const double* __restrict__ src, double* __
 // Local F repair on all active nodes, three_d/curved_boundary_warp3d.py:2543-2672.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double du_axis3(const double* uc, const int* nbr, int N, int n,
-                                           int qp, int qm, double h) {
+                                           int qp, int qm, const DivC& h1, const DivC& h2) {
   int pp = nbr[(size_t)qp * N + n];
   int pm = nbr[(size_t)qm * N + n];
-  if (pp >= 0 && pm >= 0) return (uc[pp] - uc[pm]) / (2.0 * h);
+  if (pp >= 0 && pm >= 0) return divc(uc[pp] - uc[pm], h2);
   if (pp >= 0) {
     int pp2 = nbr[(size_t)qp * N + pp];
-    if (pp2 >= 0) return (-3.0 * uc[n] + 4.0 * uc[pp] - uc[pp2]) / (2.0 * h);
-    return (uc[pp] - uc[n]) / h;
+    if (pp2 >= 0) return divc(-3.0 * uc[n] + 4.0 * uc[pp] - uc[pp2], h2);
+    return divc(uc[pp] - uc[n], h1);
   }
   if (pm >= 0) {
     int pm2 = nbr[(size_t)qm * N + pm];
-    if (pm2 >= 0) return (3.0 * uc[n] - 4.0 * uc[pm] + uc[pm2]) / (2.0 * h);
-    return (uc[n] - uc[pm]) / h;
+    if (pm2 >= 0) return divc(3.0 * uc[n] - 4.0 * uc[pm] + uc[pm2], h2);
+    return divc(uc[n] - uc[pm], h1);
   }
   return 0.0;
 }
@@ -206,10 +221,9 @@ __global__ void __launch_bounds__(128) k_repair3(Ctx3 c, double* __restrict__ f,
   double beta = fmax(0.0, fmin(1.0, p.blend));
   double o[9], t[9], nn[9];
   for (int k = 0; k < 9; ++k) o[k] = U[(size_t)(3 + k) * N + n];
-  const double h[3] = {p.dx, p.dy, p.dz};
   for (int comp = 0; comp < 3; ++comp)
     for (int ax = 0; ax < 3; ++ax) {
-      double g = du_axis3(u + (size_t)comp * N, p.neighbor, N, n, ax, ax + 3, h[ax]);
+      double g = du_axis3(u + (size_t)comp * N, p.neighbor, N, n, ax, ax + 3, c.h1[ax], c.h2[ax]);
       t[3 * comp + ax] = comp == ax ? 1.0 + g : g;
     }
   for (int k = 0; k < 9; ++k) nn[k] = o[k] + beta * (t[k] - o[k]);
@@ -260,9 +274,11 @@ __global__ void __launch_bounds__(256) k_stream3(Ctx3 c, const double* __restric
 // ---------------------------------------------------------------------------
 // three_d/curved_boundary_warp3d.py:2755-2809 (_local_characteristic_population3)
 __device__ void char_population3(const double* Ub, const double* Gx, const double* Gy,
-                                 const double* Gz, const double* d, double eta, double dt,
-                                 double c, const cvlbm3d_problem& p, const Mat& m, double omega,
+                                 const double* Gz, const double* d, double eta, const Ctx3& cx,
                                  double* out) {
+  const cvlbm3d_problem& p = cx.p;
+  const Mat& m = cx.m;
+  const double dt = p.dt, c = p.c, omega = p.omega;
   double dG[12], shift[12];
   const double k = eta * dt * c;
   for (int a = 0; a < 12; ++a) {
@@ -300,7 +316,9 @@ __device__ void char_population3(const double* Ub, const double* Gx, const doubl
   const double kk = dt / omega;
   const double kb = dt * (1.0 / omega - 0.5);
   for (int a = 0; a < 12; ++a)
-    out[a] = (Uc[a] + s3 * fl[a] / c - kk * (w[a] + s3 * Aw[a] / c) + kb * B[a]) / 6.0;
+    out[a] = divc(Uc[a] + divc(s3 * fl[a], cx.dc) - kk * (w[a] + divc(s3 * Aw[a], cx.dc)) +
+                      kb * B[a],
+                  cx.d6);
 }
 
 __device__ void link3(const Ctx3& c, int ell, const double* __restrict__ src,
@@ -419,24 +437,23 @@ __device__ void link3(const Ctx3& c, int ell, const double* __restrict__ src,
   // BFL rows (_sparse_apply_links, :3154-3241)
   if (p.recon == 1) eta = 0.5;
   const double din[3] = {(double)dx3(qi), (double)dy3(qi), (double)dz3(qi)};
-  const double cc = p.c;
   for (int a = 0; a < 12; ++a) {
     int row = a < 3 ? a : (a - 3) / 3;
     double D = 1.0, S = 0.0;
     if (ck[row] == kDirichlet) {
       if (a < 3) {
         D = -1.0;
-        S = T[a] / 3.0;
+        S = divc(T[a], c.d3);
       } else {
         int col = (a - 3) - row * 3;
-        S = -din[col] * T[row] / cc;
+        S = divc(-din[col] * T[row], c.dc);
       }
     } else {
       if (a < 3) {
-        S = -(din[0] * Pb[3 * a] + din[1] * Pb[3 * a + 1] + din[2] * Pb[3 * a + 2]) / cc;
+        S = divc(-(din[0] * Pb[3 * a] + din[1] * Pb[3 * a + 1] + din[2] * Pb[3 * a + 2]), c.dc);
       } else {
         D = -1.0;
-        S = Fb[a - 3] / 3.0;
+        S = divc(Fb[a - 3], c.d3);
       }
     }
     double fo = src[(size_t)(qo * 12 + a) * N + n];
@@ -460,7 +477,7 @@ __device__ void link3(const Ctx3& c, int ell, const double* __restrict__ src,
     for (int k = 0; k < 9; ++k) Ub[3 + k] = Fb[k];
     if (state_det3(Ub) <= m.jf) *invalid = 1;
     double out[12];
-    char_population3(Ub, G[1], G[2], G[3], din, p.link_eta[ell], p.dt, cc, p, m, p.omega, out);
+    char_population3(Ub, G[1], G[2], G[3], din, p.link_eta[ell], c, out);
     for (int a = 0; a < 12; ++a) {
       int row = a < 3 ? a : (a - 3) / 3;
       if (ck[row] == kNeumann) dst[(size_t)(qi * 12 + a) * N + n] = out[a];
@@ -496,14 +513,7 @@ __global__ void __launch_bounds__(256) k_refresh3(Ctx3 c, const double* __restri
     S[a] = s;
   }
   const double hdt = 0.5 * p.dt;
-  if (p.source_mode == kSrcConstant) {
-    for (int a = 0; a < kC3; ++a) S[a] += hdt * p.source[a];
-  } else if (p.source_mode == kSrcDamping) {
-    double den = 1.0 + hdt * p.source[0];
-    S[0] = S[0] / den;
-    S[1] = S[1] / den;
-    S[2] = S[2] / den;
-  }
+  source_half3(c, S);
   for (int a = 0; a < kC3; ++a) U[(size_t)a * N + n] = S[a];
   for (int d = 0; d < 3; ++d) u[(size_t)d * N + n] = ustar[(size_t)d * N + n] + hdt * S[d];
   if (det3(S[3], S[4], S[5], S[6], S[7], S[8], S[9], S[10], S[11]) <= c.m.jf) *invalid = 1;
@@ -615,6 +625,19 @@ Ctx3 make_ctx(const cvlbm3d_problem* p) {
   c.p = *p;
   c.m = Mat{p->mat.model, p->mat.lam, p->mat.mu, p->mat.p0, p->mat.p1, p->mat.p2, p->mat.j_floor};
   c.N = p->n_active;
+  c.hdt = 0.5 * p->dt;
+  c.k3c = 3.0 / p->c;
+  c.ff = 0.5 / p->c;
+  c.sw = p->dt * (2.0 - p->omega) * (1.0 / 12.0);
+  c.dden = make_divc(p->source_mode == kSrcDamping ? 1.0 + c.hdt * p->source[0] : 1.0);
+  const double h[3] = {p->dx, p->dy, p->dz};
+  for (int k = 0; k < 3; ++k) {
+    c.h1[k] = make_divc(h[k]);
+    c.h2[k] = make_divc(2.0 * h[k]);
+  }
+  c.d6 = make_divc(6.0);
+  c.dc = make_divc(p->c);
+  c.d3 = make_divc(3.0);
   return c;
 }
 

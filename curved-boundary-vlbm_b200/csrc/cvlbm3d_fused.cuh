@@ -47,8 +47,9 @@ struct Fused3 {
 
 // Moments with the collision's damping/source half step
 // (three_d/curved_boundary_warp3d.py:2192-2260), summed over q in order.
-__device__ __forceinline__ void moments3(const cvlbm3d_problem& p, const double* __restrict__ f,
-                                         int N, int n, double* S) {
+__device__ __forceinline__ void moments3(const Ctx3& c, const double* __restrict__ f, int n,
+                                         double* S) {
+  const int N = c.N;
 #pragma unroll
   for (int a = 0; a < kC3; ++a) {
     double s = 0.0;
@@ -56,16 +57,7 @@ __device__ __forceinline__ void moments3(const cvlbm3d_problem& p, const double*
     for (int q = 0; q < kQ3; ++q) s += f[(size_t)(q * kC3 + a) * N + n];
     S[a] = s;
   }
-  const double hdt = 0.5 * p.dt;
-  if (p.source_mode == kSrcConstant) {
-#pragma unroll
-    for (int a = 0; a < kC3; ++a) S[a] += hdt * p.source[a];
-  } else if (p.source_mode == kSrcDamping) {
-    const double den = 1.0 + hdt * p.source[0];
-    S[0] = S[0] / den;
-    S[1] = S[1] / den;
-    S[2] = S[2] / den;
-  }
+  source_half3(c, S);
 }
 
 __device__ __forceinline__ void moments_node3(const Ctx3& c, const double* __restrict__ f0,
@@ -115,7 +107,7 @@ __device__ __forceinline__ void moments_node3(const Ctx3& c, const double* __res
   const int N = c.N;
   const cvlbm3d_problem& p = c.p;
   double S[kC3];
-  moments3(p, f0, N, n, S);
+  moments3(c, f0, n, S);
 #pragma unroll
   for (int a = 0; a < kC3; ++a) U[(size_t)a * N + n] = S[a];
   const double hdt = 0.5 * p.dt;
@@ -211,7 +203,7 @@ __device__ __forceinline__ void sweep_node3(const Ctx3& c, const double* U, cons
   for (int comp = 0; comp < 3; ++comp) {
     const double uo = ldx<CG>(ucol + (size_t)comp * N + n);
     double un = uo;
-    if (d[comp] > 0.0) un = uo + p.relax * (r[comp] / d[comp] - uo);
+    if (d[comp] > 0.0) un = uo + p.relax * (sweep_quot3(c, r[comp], d[comp]) - uo);
     u[(size_t)comp * N + n] = un;
     ustar[(size_t)comp * N + n] = (uo + hdt * ldx<CG>(U + (size_t)comp * N + n)) + (un - uo);
   }
@@ -315,8 +307,7 @@ __global__ void __launch_bounds__(kQ3 * kCN, 4)
     if (p.source_mode == kSrcConstant) {
       sacc += hdt * p.source[a];
     } else if (p.source_mode == kSrcDamping && a < 3) {
-      const double den = 1.0 + hdt * p.source[0];
-      sacc = sacc / den;
+      sacc = divc(sacc, c.dden);
     }
     sm.S[a][l] = sacc;
   }
@@ -324,28 +315,27 @@ __global__ void __launch_bounds__(kQ3 * kCN, 4)
     // derivative of the swept u along each axis, as du_axis3: centred with
     // both neighbours, second-order one-sided with two on one side, first
     // order with one, zero with none
-    const double h[3] = {p.dx, p.dy, p.dz};
     for (int t = threadIdx.x; t < 9 * kCN; t += blockDim.x) {
       const int k = t / kCN, l = t % kCN, comp = k / 3, ax = k % 3;
       const int pp = sm.nb[ax][l], pm = sm.nb[ax + 3][l];
       const double* uc = u + (size_t)comp * N;
-      const double hh = h[ax];
+      const DivC &h1 = c.h1[ax], &h2 = c.h2[ax];
       double g = 0.0;
       if (n0 + l < N) {
         if (pp >= 0 && pm >= 0) {
-          g = (sm.un[ax][comp][l] - sm.un[ax + 3][comp][l]) / (2.0 * hh);
+          g = divc(sm.un[ax][comp][l] - sm.un[ax + 3][comp][l], h2);
         } else if (pp >= 0) {
           const int pp2 = p.neighbor[(size_t)ax * N + pp];
           if (pp2 >= 0)
-            g = (-3.0 * sm.u0[comp][l] + 4.0 * sm.un[ax][comp][l] - uc[pp2]) / (2.0 * hh);
+            g = divc(-3.0 * sm.u0[comp][l] + 4.0 * sm.un[ax][comp][l] - uc[pp2], h2);
           else
-            g = (sm.un[ax][comp][l] - sm.u0[comp][l]) / hh;
+            g = divc(sm.un[ax][comp][l] - sm.u0[comp][l], h1);
         } else if (pm >= 0) {
           const int pm2 = p.neighbor[(size_t)(ax + 3) * N + pm];
           if (pm2 >= 0)
-            g = (3.0 * sm.u0[comp][l] - 4.0 * sm.un[ax + 3][comp][l] + uc[pm2]) / (2.0 * hh);
+            g = divc(3.0 * sm.u0[comp][l] - 4.0 * sm.un[ax + 3][comp][l] + uc[pm2], h2);
           else
-            g = (sm.u0[comp][l] - sm.un[ax + 3][comp][l]) / hh;
+            g = divc(sm.u0[comp][l] - sm.un[ax + 3][comp][l], h1);
         }
       }
       sm.T[k][l] = comp == ax ? 1.0 + g : g;
@@ -481,7 +471,6 @@ __device__ __forceinline__ void node_prologue3(const Ctx3& c, const Fused3& fz, 
     // I + grad u of the swept u, as du_axis3: centred with both neighbours,
     // second-order one-sided with two on one side, first order with one,
     // zero with none
-    const double h[3] = {p.dx, p.dy, p.dz};
     double T[9];
 #pragma unroll
     for (int comp = 0; comp < 3; ++comp) {
@@ -490,22 +479,22 @@ __device__ __forceinline__ void node_prologue3(const Ctx3& c, const Fused3& fz, 
 #pragma unroll
       for (int ax = 0; ax < 3; ++ax) {
         const int pp = st.nb[ax], pm = st.nb[ax + 3];
-        const double hh = h[ax];
+        const DivC &h1 = c.h1[ax], &h2 = c.h2[ax];
         double g = 0.0;
         if (pp >= 0 && pm >= 0) {
-          g = (ldx<CG>(uc + pp) - ldx<CG>(uc + pm)) / (2.0 * hh);
+          g = divc(ldx<CG>(uc + pp) - ldx<CG>(uc + pm), h2);
         } else if (pp >= 0) {
           const int pp2 = p.neighbor[(size_t)ax * N + pp];
           if (pp2 >= 0)
-            g = (-3.0 * u0 + 4.0 * ldx<CG>(uc + pp) - ldx<CG>(uc + pp2)) / (2.0 * hh);
+            g = divc(-3.0 * u0 + 4.0 * ldx<CG>(uc + pp) - ldx<CG>(uc + pp2), h2);
           else
-            g = (ldx<CG>(uc + pp) - u0) / hh;
+            g = divc(ldx<CG>(uc + pp) - u0, h1);
         } else if (pm >= 0) {
           const int pm2 = p.neighbor[(size_t)(ax + 3) * N + pm];
           if (pm2 >= 0)
-            g = (3.0 * u0 - 4.0 * ldx<CG>(uc + pm) + ldx<CG>(uc + pm2)) / (2.0 * hh);
+            g = divc(3.0 * u0 - 4.0 * ldx<CG>(uc + pm) + ldx<CG>(uc + pm2), h2);
           else
-            g = (u0 - ldx<CG>(uc + pm)) / hh;
+            g = divc(u0 - ldx<CG>(uc + pm), h1);
         }
         T[3 * comp + ax] = comp == ax ? 1.0 + g : g;
       }
@@ -542,15 +531,14 @@ __device__ __forceinline__ void node_prologue3(const Ctx3& c, const Fused3& fz, 
 }
 
 template <int Q>
-__device__ __forceinline__ void collide_dir3(const cvlbm3d_problem& p, const Fused3& fz,
+__device__ __forceinline__ void collide_dir3(const Ctx3& c, const Fused3& fz,
                                              const NodeState3& st,
                                              const double* __restrict__ f0,
                                              double* __restrict__ f1, int N, int n) {
   constexpr int ax = Q % 3;
   constexpr double s = Q < 3 ? 1.0 : -1.0;
-  const double k3c = 3.0 / p.c, sixth = 1.0 / 6.0, om = p.omega;
-  const double sw = p.dt * (2.0 - om) * (1.0 / 12.0);
-  const double ff = 0.5 / p.c;
+  const cvlbm3d_problem& p = c.p;
+  const double k3c = c.k3c, sixth = 1.0 / 6.0, om = p.omega, sw = c.sw, ff = c.ff;
   const int nq = st.nb[Q];
   double* dst;
   size_t stride;
@@ -603,13 +591,12 @@ __global__ void __launch_bounds__(128, MINB)
   if (n >= N) return;
   NodeState3 st;
   node_prologue3(c, fz, U, u, do_repair, store_all, n, st);
-  const cvlbm3d_problem& p = c.p;
-  collide_dir3<0>(p, fz, st, f0, f1, N, n);
-  collide_dir3<1>(p, fz, st, f0, f1, N, n);
-  collide_dir3<2>(p, fz, st, f0, f1, N, n);
-  collide_dir3<3>(p, fz, st, f0, f1, N, n);
-  collide_dir3<4>(p, fz, st, f0, f1, N, n);
-  collide_dir3<5>(p, fz, st, f0, f1, N, n);
+  collide_dir3<0>(c, fz, st, f0, f1, N, n);
+  collide_dir3<1>(c, fz, st, f0, f1, N, n);
+  collide_dir3<2>(c, fz, st, f0, f1, N, n);
+  collide_dir3<3>(c, fz, st, f0, f1, N, n);
+  collide_dir3<4>(c, fz, st, f0, f1, N, n);
+  collide_dir3<5>(c, fz, st, f0, f1, N, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -650,7 +637,6 @@ __global__ void __launch_bounds__(128, MINB)
   int* ticket = wv.sync;
   int* timeout = wv.sync + 1;
   int* done = wv.sync + 2;
-  const cvlbm3d_problem& p = c.p;
   const int N = c.N;
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(ticket, 1);
@@ -691,12 +677,12 @@ __global__ void __launch_bounds__(128, MINB)
       } else {
         NodeState3 st;
         node_prologue3<true>(c, fz, U, u, do_repair, store_all, n, st);
-        collide_dir3<0>(p, fz, st, f0, f1, N, n);
-        collide_dir3<1>(p, fz, st, f0, f1, N, n);
-        collide_dir3<2>(p, fz, st, f0, f1, N, n);
-        collide_dir3<3>(p, fz, st, f0, f1, N, n);
-        collide_dir3<4>(p, fz, st, f0, f1, N, n);
-        collide_dir3<5>(p, fz, st, f0, f1, N, n);
+        collide_dir3<0>(c, fz, st, f0, f1, N, n);
+        collide_dir3<1>(c, fz, st, f0, f1, N, n);
+        collide_dir3<2>(c, fz, st, f0, f1, N, n);
+        collide_dir3<3>(c, fz, st, f0, f1, N, n);
+        collide_dir3<4>(c, fz, st, f0, f1, N, n);
+        collide_dir3<5>(c, fz, st, f0, f1, N, n);
       }
     }
     __threadfence();
@@ -951,25 +937,25 @@ __global__ void __launch_bounds__(128)
   double eta = p.link_eta[ell];
   if (p.recon == 1) eta = 0.5;
   const double din[3] = {(double)dx3(qi), (double)dy3(qi), (double)dz3(qi)};
-  const double cc = p.c;
   double D = 1.0, S = 0.0;
   if (ckr == kDirichlet) {
     const double Tr = fl.link_bv[(size_t)row * L + ell];
     if (a < 3) {
       D = -1.0;
-      S = fl.link_bv[(size_t)a * L + ell] / 3.0;
+      S = divc(fl.link_bv[(size_t)a * L + ell], c.d3);
     } else {
       const int col = (a - 3) - row * 3;
-      S = -din[col] * Tr / cc;
+      S = divc(-din[col] * Tr, c.dc);
     }
   } else {
     if (a < 3) {
       const double* Pb = fl.link_Pb;
-      S = -(din[0] * Pb[(size_t)(3 * a) * L + ell] + din[1] * Pb[(size_t)(3 * a + 1) * L + ell] +
-            din[2] * Pb[(size_t)(3 * a + 2) * L + ell]) / cc;
+      S = divc(-(din[0] * Pb[(size_t)(3 * a) * L + ell] + din[1] * Pb[(size_t)(3 * a + 1) * L + ell] +
+                 din[2] * Pb[(size_t)(3 * a + 2) * L + ell]),
+               c.dc);
     } else {
       D = -1.0;
-      S = fl.link_Fb[(size_t)(a - 3) * L + ell] / 3.0;
+      S = divc(fl.link_Fb[(size_t)(a - 3) * L + ell], c.d3);
     }
   }
   const double fo = fz.scratch[(size_t)ell * kC3 + a];
@@ -1010,7 +996,7 @@ __global__ void __launch_bounds__(64)
   for (int d = 0; d < 3; ++d)
     for (int a = 0; a < 12; ++a) G[d][a] = fl.char_state[((size_t)(1 + d) * 12 + a) * L + ell];
   double out[12];
-  char_population3(Ub, G[0], G[1], G[2], din, p.link_eta[ell], p.dt, p.c, p, m, p.omega, out);
+  char_population3(Ub, G[0], G[1], G[2], din, p.link_eta[ell], c, out);
   for (int a = 0; a < 12; ++a) {
     const int row = a < 3 ? a : (a - 3) / 3;
     if (ck[row] == kNeumann) f1[(size_t)(qi * kC3 + a) * N + n] = out[a];

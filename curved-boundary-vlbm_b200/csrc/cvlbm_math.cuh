@@ -37,6 +37,76 @@ struct Mat {
   double lam, mu, p0, p1, p2, jf;
 };
 
+// ---------------------------------------------------------------------------
+// Quotients by a divisor that is used more than once.
+//
+// y = RN(1/b) and e = RN((1 - b y) y) give 1/b to about 106 bits, so
+// q = RN(a y + RN(a e)) is a faithful quotient, its remainder a - b q is exact in
+// one FMA, and RN(q + (a - b q) y) is the correctly rounded a/b (Markstein 1990,
+// theorem on a faithful q and a correctly rounded reciprocal; Brisebarre, Muller
+// and Raina 2004 for known divisors).  The bits are those of a / b - checked
+// against it by the tests - at four FP64 operations instead of a reciprocal
+// sequence, range checks and branches per division: the D2Q4 node kernel makes
+// about 20 such divisions per node and the D3Q6 one 29.  Outside a safe range
+// of exponents (and for infinities and NaN) the division itself runs.  A quotient
+// below about 1e-270 may differ in its last place (the remainder is subnormal);
+// every kernel forms its quotients here, so they agree with one another.
+// ---------------------------------------------------------------------------
+CV_DEV uint32_t mag_hi(double a) { return (uint32_t)__double2hiint(a) & 0x7fffffffu; }
+
+CV_DEV double quot(double a, double b, double y, double e) {
+  const double q = fma(a, y, a * e);
+  return fma(fma(-b, q, a), y, q);
+}
+
+// A divisor known on the host (per-problem constant).
+struct DivC {
+  double b, y, e;
+  uint32_t lim;  // numerators with a smaller high word take the short form; 0: none do
+};
+
+inline DivC make_divc(double b) {
+  DivC d;
+  d.b = b;
+  d.y = 1.0 / b;
+  d.e = ::fma(-b, d.y, 1.0) * d.y;
+  const double m = ::fabs(b);
+  d.lim = (m >= 7.9e-31 && m <= 1.2e30) ? 0x78300000u : 0u;  // 2^-100 .. 2^100; |a| < 2^900
+  return d;
+}
+
+CV_DEV double divc(double a, const DivC& d) {
+  if (mag_hi(a) < d.lim) return quot(a, d.b, d.y, d.e);
+  return a / d.b;
+}
+
+// A divisor formed in the kernel, shared by several numerators of moderate size
+// (cofactors over their determinant, differences over a step): the short form is
+// used when the divisor lies in 2^-100 .. 2^100.
+struct Rcp {
+  double b, y, e;
+  bool ok;
+};
+
+CV_DEV Rcp rcp_of(double b) {
+  Rcp r;
+  r.b = b;
+  r.y = 1.0 / b;
+  r.e = fma(-b, r.y, 1.0) * r.y;
+  r.ok = mag_hi(b) - 0x39b00000u < 0x46300000u - 0x39b00000u;
+  return r;
+}
+
+CV_DEV void div_n(const Rcp& r, const double* a, double* out, int n) {
+  if (r.ok) {
+#pragma unroll
+    for (int k = 0; k < n; ++k) out[k] = quot(a[k], r.b, r.y, r.e);
+  } else {
+#pragma unroll
+    for (int k = 0; k < n; ++k) out[k] = a[k] / r.b;
+  }
+}
+
 CV_DEV double clamp_j(double j, double fl) { return j < fl ? fl : j; }
 
 // ---------------------------------------------------------------------------
@@ -64,10 +134,10 @@ CV_DEV P2 piola2(double F11, double F12, double F21, double F22, const Mat& m) {
             F21 * S01 + F22 * S11};
   }
   double J = clamp_j(F11 * F22 - F12 * F21, m.jf);
-  double H00 = F22 / J;
-  double H01 = -F21 / J;
-  double H10 = -F12 / J;
-  double H11 = F11 / J;
+  const double cof[4] = {F22, -F21, -F12, F11};
+  double H[4];
+  div_n(rcp_of(J), cof, H, 4);
+  const double H00 = H[0], H01 = H[1], H10 = H[2], H11 = H[3];
   if (m.model == kMatNeoHooke) {
     double vol = 0.5 * lam * (J * J - 1.0);
     return {mu * (F11 - H00) + vol * H00, mu * (F12 - H01) + vol * H01,
@@ -169,16 +239,11 @@ CV_DEV M3 piola3(const double* F, const Mat& m) {
     return P;
   }
   double J = clamp_j(det3(F11, F12, F13, F21, F22, F23, F31, F32, F33), m.jf);
+  const double cof[9] = {F22 * F33 - F23 * F32, F23 * F31 - F21 * F33, F21 * F32 - F22 * F31,
+                         F13 * F32 - F12 * F33, F11 * F33 - F13 * F31, F12 * F31 - F11 * F32,
+                         F12 * F23 - F13 * F22, F13 * F21 - F11 * F23, F11 * F22 - F12 * F21};
   double H[9];
-  H[0] = (F22 * F33 - F23 * F32) / J;
-  H[1] = (F23 * F31 - F21 * F33) / J;
-  H[2] = (F21 * F32 - F22 * F31) / J;
-  H[3] = (F13 * F32 - F12 * F33) / J;
-  H[4] = (F11 * F33 - F13 * F31) / J;
-  H[5] = (F12 * F31 - F11 * F32) / J;
-  H[6] = (F12 * F23 - F13 * F22) / J;
-  H[7] = (F13 * F21 - F11 * F23) / J;
-  H[8] = (F11 * F22 - F12 * F21) / J;
+  div_n(rcp_of(J), cof, H, 9);
   if (m.model == kMatNeoHooke) {
     double vol = 0.5 * lam * (J * J - 1.0);
 #pragma unroll
@@ -282,7 +347,10 @@ CV_DEV void piola3_row(const double* F, const Mat& m, int r, double* out) {
     c1 = F13 * F21 - F11 * F23;
     c2 = F11 * F22 - F12 * F21;
   }
-  const double h0 = c0 / J, h1 = c1 / J, h2 = c2 / J;
+  const double cof[3] = {c0, c1, c2};
+  double h[3];
+  div_n(rcp_of(J), cof, h, 3);
+  const double h0 = h[0], h1 = h[1], h2 = h[2];
   const double vol = 0.5 * m.lam * (J * J - 1.0);
   out[0] = m.mu * (F[3 * r] - h0) + vol * h0;
   out[1] = m.mu * (F[3 * r + 1] - h1) + vol * h1;
@@ -634,7 +702,10 @@ CV_DEV void solve_normal_image2(const double* Fg, double nx, double ny, double t
       double F21 = hn1 * nx + gt1 * tanx;
       double F22 = hn1 * ny + gt1 * tany;
       double J = clamp_j(F11 * F22 - F12 * F21, jf);
-      double H00 = F22 / J, H01 = -F21 / J, H10 = -F12 / J, H11 = F11 / J;
+      const double cof[4] = {F22, -F21, -F12, F11};
+      double H[4];
+      div_n(rcp_of(J), cof, H, 4);
+      const double H00 = H[0], H01 = H[1], H10 = H[2], H11 = H[3];
       double beta = 0.5 * lam * (J * J - 1.0) - mu;
       double coeff = lam * J * J - beta;
       double n2 = nx * nx + ny * ny;
@@ -701,11 +772,26 @@ CV_DEV void flux2_jvp(const double* U, const double* W, const Mat& m, double* Ax
   }
   P2 Pp = piola2(Up[2], Up[3], Up[4], Up[5], m);
   P2 Pm = piola2(Um[2], Um[3], Um[4], Um[5], m);
-  double den = 2.0 * eps;
-  for (int a = 0; a < 6; ++a) {
-    AxW[a] = (flux2x(a, Up, Pp) - flux2x(a, Um, Pm)) / den;
-    AyW[a] = (flux2y(a, Up, Pp) - flux2y(a, Um, Pm)) / den;
-  }
+  // the x flux has no rows 3 and 5, the y flux no rows 2 and 4: 0 / den = 0
+  const double num[8] = {
+      flux2x(0, Up, Pp) - flux2x(0, Um, Pm), flux2x(1, Up, Pp) - flux2x(1, Um, Pm),
+      flux2x(2, Up, Pp) - flux2x(2, Um, Pm), flux2x(4, Up, Pp) - flux2x(4, Um, Pm),
+      flux2y(0, Up, Pp) - flux2y(0, Um, Pm), flux2y(1, Up, Pp) - flux2y(1, Um, Pm),
+      flux2y(3, Up, Pp) - flux2y(3, Um, Pm), flux2y(5, Up, Pp) - flux2y(5, Um, Pm)};
+  double d[8];
+  div_n(rcp_of(2.0 * eps), num, d, 8);
+  AxW[0] = d[0];
+  AxW[1] = d[1];
+  AxW[2] = d[2];
+  AxW[3] = 0.0;
+  AxW[4] = d[3];
+  AxW[5] = 0.0;
+  AyW[0] = d[4];
+  AyW[1] = d[5];
+  AyW[2] = 0.0;
+  AyW[3] = d[6];
+  AyW[4] = 0.0;
+  AyW[5] = d[7];
 }
 
 // ---------------------------------------------------------------------------
@@ -827,15 +913,12 @@ CV_DEV void solve_Fb3(const double* Fg, double nx, double ny, double nz, const d
       double J = det3v(F);
       if (J < m.jf) J = m.jf;
       double H[9];
-      H[0] = (F[4] * F[8] - F[5] * F[7]) / J;
-      H[1] = (F[5] * F[6] - F[3] * F[8]) / J;
-      H[2] = (F[3] * F[7] - F[4] * F[6]) / J;
-      H[3] = (F[2] * F[7] - F[1] * F[8]) / J;
-      H[4] = (F[0] * F[8] - F[2] * F[6]) / J;
-      H[5] = (F[1] * F[6] - F[0] * F[7]) / J;
-      H[6] = (F[1] * F[5] - F[2] * F[4]) / J;
-      H[7] = (F[2] * F[3] - F[0] * F[5]) / J;
-      H[8] = (F[0] * F[4] - F[1] * F[3]) / J;
+      const double cof[9] = {F[4] * F[8] - F[5] * F[7], F[5] * F[6] - F[3] * F[8],
+                             F[3] * F[7] - F[4] * F[6], F[2] * F[7] - F[1] * F[8],
+                             F[0] * F[8] - F[2] * F[6], F[1] * F[6] - F[0] * F[7],
+                             F[1] * F[5] - F[2] * F[4], F[2] * F[3] - F[0] * F[5],
+                             F[0] * F[4] - F[1] * F[3]};
+      div_n(rcp_of(J), cof, H, 9);
       double beta = 0.5 * m.lam * (J * J - 1.0) - m.mu;
       double coeff = m.lam * J * J - beta;
       double n2 = fr.n[0] * fr.n[0] + fr.n[1] * fr.n[1] + fr.n[2] * fr.n[2];
@@ -859,12 +942,13 @@ CV_DEV void solve_Fb3(const double* Fg, double nx, double ny, double nz, const d
                  hh = A[7], ii = A[8];
     double det = a * (e * ii - f * hh) - b * (d * ii - f * g) + c * (d * hh - e * g);
     if (fabs(det) < 1.0e-14) break;
-    double i00 = (e * ii - f * hh) / det, i01 = (c * hh - b * ii) / det,
-           i02 = (b * f - c * e) / det;
-    double i10 = (f * g - d * ii) / det, i11 = (a * ii - c * g) / det,
-           i12 = (c * d - a * f) / det;
-    double i20 = (d * hh - e * g) / det, i21 = (b * g - a * hh) / det,
-           i22 = (a * e - b * d) / det;
+    const double adj[9] = {e * ii - f * hh, c * hh - b * ii, b * f - c * e,
+                           f * g - d * ii, a * ii - c * g, c * d - a * f,
+                           d * hh - e * g, b * g - a * hh, a * e - b * d};
+    double inv[9];
+    div_n(rcp_of(det), adj, inv, 9);
+    const double i00 = inv[0], i01 = inv[1], i02 = inv[2], i10 = inv[3], i11 = inv[4],
+                 i12 = inv[5], i20 = inv[6], i21 = inv[7], i22 = inv[8];
     double dl[3] = {-(i00 * r[0] + i01 * r[1] + i02 * r[2]),
                     -(i10 * r[0] + i11 * r[1] + i12 * r[2]),
                     -(i20 * r[0] + i21 * r[1] + i22 * r[2])};
@@ -967,15 +1051,12 @@ CV_DEV void solve_Fb3_mixed(const double* Fg, double nx, double ny, double nz, c
       double J = det3v(F);
       if (J < m.jf) J = m.jf;
       double H[9];
-      H[0] = (F[4] * F[8] - F[5] * F[7]) / J;
-      H[1] = (F[5] * F[6] - F[3] * F[8]) / J;
-      H[2] = (F[3] * F[7] - F[4] * F[6]) / J;
-      H[3] = (F[2] * F[7] - F[1] * F[8]) / J;
-      H[4] = (F[0] * F[8] - F[2] * F[6]) / J;
-      H[5] = (F[1] * F[6] - F[0] * F[7]) / J;
-      H[6] = (F[1] * F[5] - F[2] * F[4]) / J;
-      H[7] = (F[2] * F[3] - F[0] * F[5]) / J;
-      H[8] = (F[0] * F[4] - F[1] * F[3]) / J;
+      const double cof[9] = {F[4] * F[8] - F[5] * F[7], F[5] * F[6] - F[3] * F[8],
+                             F[3] * F[7] - F[4] * F[6], F[2] * F[7] - F[1] * F[8],
+                             F[0] * F[8] - F[2] * F[6], F[1] * F[6] - F[0] * F[7],
+                             F[1] * F[5] - F[2] * F[4], F[2] * F[3] - F[0] * F[5],
+                             F[0] * F[4] - F[1] * F[3]};
+      div_n(rcp_of(J), cof, H, 9);
       const double beta = 0.5 * m.lam * (J * J - 1.0) - m.mu;
       const double coeff = m.lam * J * J - beta;
       const double n2 = fr.n[0] * fr.n[0] + fr.n[1] * fr.n[1] + fr.n[2] * fr.n[2];
@@ -1002,12 +1083,13 @@ CV_DEV void solve_Fb3_mixed(const double* Fg, double nx, double ny, double nz, c
                  hh = A[7], ii = A[8];
     const double det = a * (e * ii - f * hh) - b * (d * ii - f * g) + c * (d * hh - e * g);
     if (fabs(det) < 1.0e-14) break;
-    const double i00 = (e * ii - f * hh) / det, i01 = (c * hh - b * ii) / det,
-                 i02 = (b * f - c * e) / det;
-    const double i10 = (f * g - d * ii) / det, i11 = (a * ii - c * g) / det,
-                 i12 = (c * d - a * f) / det;
-    const double i20 = (d * hh - e * g) / det, i21 = (b * g - a * hh) / det,
-                 i22 = (a * e - b * d) / det;
+    const double adj[9] = {e * ii - f * hh, c * hh - b * ii, b * f - c * e,
+                           f * g - d * ii, a * ii - c * g, c * d - a * f,
+                           d * hh - e * g, b * g - a * hh, a * e - b * d};
+    double inv[9];
+    div_n(rcp_of(det), adj, inv, 9);
+    const double i00 = inv[0], i01 = inv[1], i02 = inv[2], i10 = inv[3], i11 = inv[4],
+                 i12 = inv[5], i20 = inv[6], i21 = inv[7], i22 = inv[8];
     const double dl[3] = {-(i00 * rm[0] + i01 * rm[1] + i02 * rm[2]),
                           -(i10 * rm[0] + i11 * rm[1] + i12 * rm[2]),
                           -(i20 * rm[0] + i21 * rm[1] + i22 * rm[2])};
@@ -1043,8 +1125,11 @@ CV_DEV void jvp3(int axis, const double* U, const double* W, const Mat& m, doubl
   M3 Pp = piola3(Fp, m);
   M3 Pm = piola3(Fm, m);
   for (int a = 0; a < 12; ++a) out[a] = 0.0;
+  double num[3], dq[3];
+  for (int i = 0; i < 3; ++i) num[i] = -(Pp.v[3 * i + axis] - Pm.v[3 * i + axis]);
+  div_n(rcp_of(2.0 * eps), num, dq, 3);
   for (int i = 0; i < 3; ++i) {
-    out[i] = -(Pp.v[3 * i + axis] - Pm.v[3 * i + axis]) / (2.0 * eps);
+    out[i] = dq[i];
     out[3 + 3 * i + axis] = -W[i];
   }
 }
