@@ -530,6 +530,7 @@ __global__ void k_set_ustar3(int N, const double* __restrict__ disp, const doubl
 }  // namespace
 
 #include "cvlbm3d_fused.cuh"
+#include "cvlbm3d_links.cuh"
 
 namespace {
 
@@ -665,6 +666,14 @@ extern "C" int cvlbm3d_run(const cvlbm3d_problem* p, cvlbm3d_fields* f, double t
     // U and u_next.  So they run on a second stream after the collide of step
     // k, while the links do; the moments of the link nodes follow the links.
     const bool wave = wave_ok3(p, f) && N > 0;
+    const bool packed = p->char_packed && p->char_slot_lm && p->char_w_lm;
+    const LinkFn3 link_fn = link_finish3(c.m.model);
+    const CollideFn3 collide_fn = p->node_variant == 1   ? collide3<3>(c.m.model)
+                                  : p->node_variant == 2 ? collide3<5>(c.m.model)
+                                                         : collide3<4>(c.m.model);
+    if (kCollideSmem3 > 48 * 1024)
+      cudaFuncSetAttribute(collide_fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kCollideSmem3);
     Overlap3* ov = nullptr;
     if (!wave && p->overlap && p->disp_interval == 1 && N > 0 && L > 0 && p->link_nodes &&
         p->n_link_nodes > 0 && nsteps > 1)
@@ -702,15 +711,8 @@ extern "C" int cvlbm3d_run(const cvlbm3d_problem* p, cvlbm3d_fields* f, double t
           k3_sweep<<<blocks(N, 256), 256, 0, s>>>(c, f->U, f->u_next, f->u, f->u_star, clock, t);
           cv::count_launches(1);
         }
-        if (p->node_variant == 1)
-          k3_collide<<<blocks(N, kCN), kQ3 * kCN, 0, s>>>(c, fz, f->f0, f->f1, f->U, f->u,
-                                                          repair, k == nsteps - 1);
-        else if (p->node_variant == 2)
-          k3_collide_node<3><<<blocks(N, 128), 128, 0, s>>>(c, fz, f->f0, f->f1, f->U, f->u,
-                                                            repair, k == nsteps - 1);
-        else
-          k3_collide_node<4><<<blocks(N, 128), 128, 0, s>>>(c, fz, f->f0, f->f1, f->U, f->u,
-                                                            repair, k == nsteps - 1);
+        collide_fn<<<blocks(N, kCT3), kCT3, kCollideSmem3, s>>>(c, fz, f->f0, f->f1, f->U, f->u,
+                                                                repair, k == nsteps - 1);
         cv::count_launches(1);
         if (ov && k + 1 < nsteps) {
           // a sweep is due every step, so these moments write u_next
@@ -723,9 +725,13 @@ extern "C" int cvlbm3d_run(const cvlbm3d_problem* p, cvlbm3d_fields* f, double t
         }
       }
       timer_end(tk, s);
-      if (L > 0) {
+      if (L > 0 && p->has_char && packed) {
+        k3_link_gather_packed<<<blocks(L, kLinks3), kLT3, 0, s>>>(c, fz, f->char_state);
+        link_fn<<<blocks(L, kFinish3), kFinish3, 0, s>>>(c, fz, f->f1, f->u, *f, clock, t, 0.5 * p->dt);
+        cv::count_launches(2);
+      } else if (L > 0) {
         if (p->has_char) {
-          if (p->char_slot_lm && p->char_w_lm)
+          if (p->char_slot_lm && p->char_w_lm && !p->char_packed)
             k3_link_gather4<<<blocks(L, kGather4Links), 128, 0, s>>>(c, fz, f->char_state);
           else
             k3_link_gather<<<blocks(L, kGatherLinks), 128, 0, s>>>(c, fz, f->char_state);

@@ -6,14 +6,12 @@
 //                (u_next), invalid flag; when no sweep is due, u and u* too
 //   k3_sweep     u_swept -> u and the trapezoidal u* update, from U and ucol
 //                of the node and its six neighbours plus cut-point anchors
-//   k3_collide_node (default; one thread per node) or k3_collide (six
-//                warps per 32 nodes, one per direction; shared memory):
-//                f0 again, F repair from the swept u (+-2 star stencil), BGK
-//                collision with damping/source, repair delta and push
-//                streaming to f1; a population whose neighbour is not active
-//                leaves through a cut link and is kept per link
-//                (link_scratch) for the link kernels; the post-step U of
-//                nodes that links read goes to U_need, one 96-byte row each
+//   k3_collide   one thread per node: F repair from the swept u (+-2 star
+//                stencil), f0 again, BGK collision with damping/source, repair
+//                delta and push streaming to f1; a population whose neighbour
+//                is not active leaves through a cut link and is kept per link
+//                (link_scratch) for the link kernels; the post-step U of nodes
+//                that links read goes to U_need, one 96-byte row each
 //   k3_moments_part  the moments of the nodes without / with a cut link,
 //                for the optional overlap of the next step with the links
 // Per active node this reads f0 twice and writes f1 once (the f0 re-read of
@@ -22,7 +20,8 @@
 // against the algorithmic 1.2 KB).
 //
 // Link kernels (the four phases of apply_boundary_reconstruction,
-// three_d/curved_boundary_warp3d.py:4339-4399):
+// three_d/curved_boundary_warp3d.py:4339-4399): cvlbm3d_links.cuh for problems with
+// packed characteristic tables; without them
 //   k3_link_gather   16 lanes per link, one per component: value and
 //                    gradient of the characteristic stencil (:2675-2700)
 //   k3_link_prepare  one thread per link: boundary value, F predictor, Newton
@@ -175,28 +174,48 @@ __device__ __forceinline__ void sweep_node3(const Ctx3& c, const double* U, cons
   double Fs[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) Fs[k] = ldx<CG>(Ub + (size_t)k * N + n);
+  int nb[kQ3];
 #pragma unroll
-  for (int q = 0; q < kQ3; ++q) {
-    const int m = p.neighbor[(size_t)q * N + n];
-    if (m < 0) continue;
-    const double ddx = (double)dx3(q) * p.dx, ddy = (double)dy3(q) * p.dy,
-                 ddz = (double)dz3(q) * p.dz;
-    const double* Um = Ub + m;
-    const size_t NN = (size_t)N;
-    const double g0 = 0.5 * ((Fs[0] + ldx<CG>(Um) - 2.0) * ddx + (Fs[1] + ldx<CG>(Um + NN)) * ddy +
-                             (Fs[2] + ldx<CG>(Um + 2 * NN)) * ddz);
-    const double g1 = 0.5 * ((Fs[3] + ldx<CG>(Um + 3 * NN)) * ddx +
-                             (Fs[4] + ldx<CG>(Um + 4 * NN) - 2.0) * ddy +
-                             (Fs[5] + ldx<CG>(Um + 5 * NN)) * ddz);
-    const double g2 = 0.5 * ((Fs[6] + ldx<CG>(Um + 6 * NN)) * ddx +
-                             (Fs[7] + ldx<CG>(Um + 7 * NN)) * ddy +
-                             (Fs[8] + ldx<CG>(Um + 8 * NN) - 2.0) * ddz);
-    r[0] += ldx<CG>(ucol + m) - g0;
-    r[1] += ldx<CG>(ucol + (size_t)N + m) - g1;
-    r[2] += ldx<CG>(ucol + 2 * (size_t)N + m) - g2;
-    d[0] += 1.0;
-    d[1] += 1.0;
-    d[2] += 1.0;
+  for (int q = 0; q < kQ3; ++q) nb[q] = p.neighbor[(size_t)q * N + n];
+  // of (F_x dx + F_y dy + F_z dz) only the term on the direction's axis is formed:
+  // the other two are products with an exact zero
+  auto add = [&](int q, const double* e, const double* un) {
+    const int ax = q % 3;
+    const double h = q < 3 ? (ax == 0 ? p.dx : ax == 1 ? p.dy : p.dz)
+                           : -(ax == 0 ? p.dx : ax == 1 ? p.dy : p.dz);
+#pragma unroll
+    for (int comp = 0; comp < 3; ++comp) {
+      double v = Fs[3 * comp + ax] + e[comp];
+      if (comp == ax) v = v - 2.0;
+      r[comp] += un[comp] - 0.5 * (v * h);
+      d[comp] += 1.0;
+    }
+  };
+  if ((nb[0] | nb[1] | nb[2] | nb[3] | nb[4] | nb[5]) >= 0) {
+    // all six neighbours: their 36 values are loaded before the first is used
+    double e[kQ3][3], un[kQ3][3];
+#pragma unroll
+    for (int q = 0; q < kQ3; ++q) {
+#pragma unroll
+      for (int comp = 0; comp < 3; ++comp) {
+        e[q][comp] = ldx<CG>(Ub + (size_t)(3 * comp + q % 3) * N + nb[q]);
+        un[q][comp] = ldx<CG>(ucol + (size_t)comp * N + nb[q]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kQ3; ++q) add(q, e[q], un[q]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < kQ3; ++q) {
+      if (nb[q] < 0) continue;
+      double e[3], un[3];
+#pragma unroll
+      for (int comp = 0; comp < 3; ++comp) {
+        e[comp] = ldx<CG>(Ub + (size_t)(3 * comp + q % 3) * N + nb[q]);
+        un[comp] = ldx<CG>(ucol + (size_t)comp * N + nb[q]);
+      }
+      add(q, e, un);
+    }
   }
   const double hdt = 0.5 * p.dt;
 #pragma unroll
@@ -209,7 +228,10 @@ __device__ __forceinline__ void sweep_node3(const Ctx3& c, const double* U, cons
   }
 }
 
-__global__ void __launch_bounds__(256) k3_sweep(Ctx3 c, const double* __restrict__ U,
+// The neighbours' values are scattered loads that miss L1 at the plane neighbours:
+// bound by their latency, so warps count (four blocks of 256, 64 registers: shell176
+// 4,799 us per four steps against 4,863 with three and 5,057 with two).
+__global__ void __launch_bounds__(256, 4) k3_sweep(Ctx3 c, const double* __restrict__ U,
                                                 const double* __restrict__ ucol,
                                                 double* __restrict__ u,
                                                 double* __restrict__ ustar, const double* clock,
@@ -219,226 +241,23 @@ __global__ void __launch_bounds__(256) k3_sweep(Ctx3 c, const double* __restrict
   sweep_node3<false>(c, U, ucol, u, ustar, clock, t_host, n);
 }
 
-// Collision + F repair + push streaming (three_d/curved_boundary_warp3d.py
-// :2192-2330, 2543-2672).  `u` is the swept displacement of every node.
-//
-// A block takes 32 consecutive active nodes with six warps, warp q owning
-// direction q (lane = node), so every population load and store is one
-// coalesced 256-byte row:
-//   1  warp q loads f0[q][0..11] of its 32 nodes (kept in registers, copied
-//      to shared memory for the moments)
-//   2  moments (summed over q in order) and the nine targets of I + grad u
-//      (+-2 star stencil of the swept u), spread over the block
-//   3  P(F) and P(F_repaired), one row per warp (six rows), U / U_need rows
-//   4  warp q: collision, repair delta and push of direction q
-constexpr int kCN = 32;  // nodes per collide block (one per lane)
-
-struct CollideSmem3 {
-  double f[kQ3][kC3][kCN];
-  double un[kQ3][3][kCN];  // swept u of the neighbour in direction q
-  double u0[3][kCN];       // swept u of the node
-  int nb[kQ3][kCN];        // neighbour in direction q, -1 if not active
-  double S[kC3][kCN];
-  double T[9][kCN];   // I + grad u
-  double Po[9][kCN];  // P(F)
-  double Pn[9][kCN];  // P(F_repaired)
-  double dF[9][kCN];  // F_repaired - F
-  int rep[kCN];
-};
-
-// feq of (q, a) with the moments and P(F) of lane `l` in shared memory; the
-// same operations as feq3 (zero-weight axes included).
-__device__ __forceinline__ double feq3_smem(int q, int a, const CollideSmem3& sm, int l,
-                                            double three_over_c, double sixth) {
-  const double sx = (double)dx3(q), sy = (double)dy3(q), sz = (double)dz3(q);
-  double f0, f1, f2;
-  if (a < 3) {
-    f0 = -sm.Po[3 * a][l];
-    f1 = -sm.Po[3 * a + 1][l];
-    f2 = -sm.Po[3 * a + 2][l];
-  } else {
-    const int r = a - 3, ax = r % 3;
-    const double v = -sm.S[r / 3][l];
-    f0 = ax == 0 ? v : 0.0;
-    f1 = ax == 1 ? v : 0.0;
-    f2 = ax == 2 ? v : 0.0;
-  }
-  return sixth * (sm.S[a][l] + three_over_c * (sx * f0 + sy * f1 + sz * f2));
+// The material of a kernel: the problem's, its law fixed when compiled for one.
+template <int MAT>
+__device__ __forceinline__ Mat mat3(const Ctx3& c) {
+  Mat m = c.m;
+  if (MAT >= 0) m.model = MAT;
+  return m;
 }
 
-__global__ void __launch_bounds__(kQ3 * kCN, 4)
-    k3_collide(Ctx3 c, Fused3 fz, const double* __restrict__ f0, double* __restrict__ f1,
-               double* __restrict__ U, const double* __restrict__ u, int do_repair,
-               int store_all) {
-  __shared__ CollideSmem3 sm;
-  const int N = c.N;
-  const cvlbm3d_problem& p = c.p;
-  const Mat& m = c.m;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int n0 = blockIdx.x * kCN;
-  const int n = n0 + lane;
-  const bool live = n < N;
-
-  // 1: populations of direction `warp`, its neighbour and (for the repair)
-  // the neighbour's swept u
-  double v[kC3];
-  const int q = warp;
-#pragma unroll
-  for (int a = 0; a < kC3; ++a) v[a] = live ? f0[(size_t)(q * kC3 + a) * N + n] : 0.0;
-  const int nq = live ? p.neighbor[(size_t)q * N + n] : -1;
-  if (do_repair) {
-#pragma unroll
-    for (int comp = 0; comp < 3; ++comp)
-      sm.un[q][comp][lane] = nq >= 0 ? u[(size_t)comp * N + nq] : 0.0;
-    if (warp < 3) sm.u0[warp][lane] = live ? u[(size_t)warp * N + n] : 0.0;
-  }
-#pragma unroll
-  for (int a = 0; a < kC3; ++a) sm.f[q][a][lane] = v[a];
-  sm.nb[q][lane] = nq;
-  __syncthreads();
-
-  // 2: moments (12 x 32 sums) and I + grad u (9 x 32 targets)
-  const double hdt = 0.5 * p.dt;
-  for (int t = threadIdx.x; t < kC3 * kCN; t += blockDim.x) {
-    const int a = t / kCN, l = t % kCN;
-    double sacc = 0.0;
-#pragma unroll
-    for (int qq = 0; qq < kQ3; ++qq) sacc += sm.f[qq][a][l];
-    if (p.source_mode == kSrcConstant) {
-      sacc += hdt * p.source[a];
-    } else if (p.source_mode == kSrcDamping && a < 3) {
-      sacc = divc(sacc, c.dden);
-    }
-    sm.S[a][l] = sacc;
-  }
-  if (do_repair) {
-    // derivative of the swept u along each axis, as du_axis3: centred with
-    // both neighbours, second-order one-sided with two on one side, first
-    // order with one, zero with none
-    for (int t = threadIdx.x; t < 9 * kCN; t += blockDim.x) {
-      const int k = t / kCN, l = t % kCN, comp = k / 3, ax = k % 3;
-      const int pp = sm.nb[ax][l], pm = sm.nb[ax + 3][l];
-      const double* uc = u + (size_t)comp * N;
-      const DivC &h1 = c.h1[ax], &h2 = c.h2[ax];
-      double g = 0.0;
-      if (n0 + l < N) {
-        if (pp >= 0 && pm >= 0) {
-          g = divc(sm.un[ax][comp][l] - sm.un[ax + 3][comp][l], h2);
-        } else if (pp >= 0) {
-          const int pp2 = p.neighbor[(size_t)ax * N + pp];
-          if (pp2 >= 0)
-            g = divc(-3.0 * sm.u0[comp][l] + 4.0 * sm.un[ax][comp][l] - uc[pp2], h2);
-          else
-            g = divc(sm.un[ax][comp][l] - sm.u0[comp][l], h1);
-        } else if (pm >= 0) {
-          const int pm2 = p.neighbor[(size_t)(ax + 3) * N + pm];
-          if (pm2 >= 0)
-            g = divc(3.0 * sm.u0[comp][l] - 4.0 * sm.un[ax + 3][comp][l] + uc[pm2], h2);
-          else
-            g = divc(sm.u0[comp][l] - sm.un[ax + 3][comp][l], h1);
-        }
-      }
-      sm.T[k][l] = comp == ax ? 1.0 + g : g;
-    }
-  }
-  __syncthreads();
-
-  // 3: P(F) and P(F_repaired), one row of each per warp: warps 0-2 row
-  // `warp` of P(F), warps 3-5 row `warp - 3` of the repaired F and its Piola;
-  // warp 3 also writes the repaired flag and the U / U_need rows
-  {
-    const int row = warp < 3 ? warp : warp - 3;
-    double F[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) F[k] = sm.S[3 + k][lane];
-    if (warp < 3) {
-      double Pr[3];
-      piola3_row(F, m, row, Pr);
-#pragma unroll
-      for (int c2 = 0; c2 < 3; ++c2) sm.Po[3 * row + c2][lane] = Pr[c2];
-    } else {
-      bool repaired = false;
-      double nn[9];
-      if (do_repair) {
-        const double beta = fmax(0.0, fmin(1.0, p.blend));
-#pragma unroll
-        for (int k = 0; k < 9; ++k) nn[k] = F[k] + beta * (sm.T[k][lane] - F[k]);
-        if (det3v(nn) > m.jf) {
-          repaired = true;
-          double Pr[3];
-          piola3_row(nn, m, row, Pr);
-#pragma unroll
-          for (int c2 = 0; c2 < 3; ++c2) {
-            sm.Pn[3 * row + c2][lane] = Pr[c2];
-            sm.dF[3 * row + c2][lane] = nn[3 * row + c2] - F[3 * row + c2];
-          }
-        }
-      }
-      if (warp == 3) {
-        sm.rep[lane] = repaired ? 1 : 0;
-        if (repaired && store_all && live) {
-#pragma unroll
-          for (int k = 0; k < 9; ++k) U[(size_t)(3 + k) * N + n] = nn[k];
-        }
-        const int slot = live ? fz.need_slot[n] : -1;
-        if (slot >= 0) {
-          double* rowp = fz.Uneed + (size_t)slot * kC3;
-          rowp[0] = sm.S[0][lane];
-          rowp[1] = sm.S[1][lane];
-          rowp[2] = sm.S[2][lane];
-#pragma unroll
-          for (int k = 0; k < 9; ++k) rowp[3 + k] = repaired ? nn[k] : F[k];
-        }
-      }
-    }
-  }
-  __syncthreads();
-  if (!live) return;
-
-  // 4: collision, repair delta, push of direction q
-  const double k3c = 3.0 / p.c, sixth = 1.0 / 6.0, om = p.omega;
-  const double sw = p.dt * (2.0 - om) * (1.0 / 12.0);
-  const double ff = 0.5 / p.c;
-  const bool repaired = sm.rep[lane] != 0;
-  int ell = -1;
-  if (nq < 0) {
-    for (int k = p.node_link_start[n]; k < p.node_link_start[n + 1]; ++k) {
-      const int e = p.node_link_list[k];
-      if (p.link_q[e] == q) ell = e;
-    }
-  }
-  const double sx = (double)dx3(q), sy = (double)dy3(q), sz = (double)dz3(q);
-  const double vel[3] = {sm.S[0][lane], sm.S[1][lane], sm.S[2][lane]};
-#pragma unroll
-  for (int a = 0; a < kC3; ++a) {
-    const double old = v[a];
-    const double fe = feq3_smem(q, a, sm, lane, k3c, sixth);
-    double val = old + om * (fe - old) + sw * source_comp3(a, p.source_mode, p.source, vel);
-    if (repaired) {
-      if (a < 3)
-        val = val - ff * (sx * (sm.Pn[3 * a][lane] - sm.Po[3 * a][lane]) +
-                          sy * (sm.Pn[3 * a + 1][lane] - sm.Po[3 * a + 1][lane]) +
-                          sz * (sm.Pn[3 * a + 2][lane] - sm.Po[3 * a + 2][lane]));
-      else
-        val = val + sixth * sm.dF[a - 3][lane];
-    }
-    if (nq >= 0)
-      f1[(size_t)(q * kC3 + a) * N + nq] = val;
-    else if (ell >= 0)
-      fz.scratch[(size_t)ell * kC3 + a] = val;
-  }
-}
-
-// Collision + F repair + push streaming, one thread per node.
+// Collision + F repair + push streaming of one node with its state in registers and
+// the six directions unrolled (the wavefront kernel's collide items).
 //
-// The moments come from U, which k3_moments wrote this step with the same
-// sums (so they equal the shared-memory sums of k3_collide bit for bit), and
-// P(F), P(F_repaired) are evaluated once per node.  Each direction is then 12
+// The moments come from U, which the moments wrote this step, and P(F), P(F_repaired) are evaluated once per node.  Each direction is then 12
 // coalesced loads of f0 and 12 stores to f1 at the neighbour, with the
 // direction a compile-time constant: of the three terms s_x f_x + s_y f_y +
 // s_z f_z of the equilibrium flux only the one on the direction's axis is
 // formed (the others are products with an exact zero, which change no finite
-// sum), so the arithmetic is that of k3_collide without its 0 * x products.
+// sum).
 struct NodeState3 {
   double S[kC3];
   double Po[9];  // P(F)
@@ -450,21 +269,23 @@ struct NodeState3 {
 
 // Moments, neighbours, P(F), the F repair and its Piola difference; the U
 // and U_need rows of the node.
-template <bool CG = false>
+template <int MAT, bool CG = false>
 __device__ __forceinline__ void node_prologue3(const Ctx3& c, const Fused3& fz, double* U,
                                                const double* u, int do_repair, int store_all,
                                                int n, NodeState3& st) {
   const int N = c.N;
   const cvlbm3d_problem& p = c.p;
-  const Mat& m = c.m;
+  const Mat m = mat3<MAT>(c);
 #pragma unroll
   for (int a = 0; a < kC3; ++a) st.S[a] = ldx<CG>(U + (size_t)a * N + n);
 #pragma unroll
   for (int q = 0; q < kQ3; ++q) st.nb[q] = p.neighbor[(size_t)q * N + n];
   const double* F = st.S + 3;
+  {
+    const M3 P = piola3(F, m);
 #pragma unroll
-  for (int r = 0; r < 3; ++r) piola3_row(F, m, r, st.Po + 3 * r);
-
+    for (int k = 0; k < 9; ++k) st.Po[k] = P.v[k];
+  }
   st.repaired = false;
   double nn[9];
   if (do_repair) {
@@ -504,15 +325,12 @@ __device__ __forceinline__ void node_prologue3(const Ctx3& c, const Fused3& fz, 
     for (int k = 0; k < 9; ++k) nn[k] = F[k] + beta * (T[k] - F[k]);
     if (det3v(nn) > m.jf) {
       st.repaired = true;
+      const M3 P = piola3(nn, m);
 #pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        double Pr[3];
-        piola3_row(nn, m, r, Pr);
-#pragma unroll
-        for (int c2 = 0; c2 < 3; ++c2) st.dP[3 * r + c2] = Pr[c2] - st.Po[3 * r + c2];
+      for (int k = 0; k < 9; ++k) {
+        st.dP[k] = P.v[k] - st.Po[k];
+        st.dF[k] = nn[k] - F[k];
       }
-#pragma unroll
-      for (int k = 0; k < 9; ++k) st.dF[k] = nn[k] - F[k];
     }
   }
   if (st.repaired && store_all) {
@@ -541,7 +359,7 @@ __device__ __forceinline__ void collide_dir3(const Ctx3& c, const Fused3& fz,
   const double k3c = c.k3c, sixth = 1.0 / 6.0, om = p.omega, sw = c.sw, ff = c.ff;
   const int nq = st.nb[Q];
   double* dst;
-  size_t stride;
+  size_t stride;  // pointers advance row by row: one 64-bit addition per access
   if (nq >= 0) {
     dst = f1 + (size_t)(Q * kC3) * N + nq;
     stride = (size_t)N;
@@ -555,9 +373,13 @@ __device__ __forceinline__ void collide_dir3(const Ctx3& c, const Fused3& fz,
     dst = fz.scratch + (size_t)ell * kC3;
     stride = 1;
   }
+  const double* src = f0 + (size_t)(Q * kC3) * N + n;
   double old[kC3];
 #pragma unroll
-  for (int a = 0; a < kC3; ++a) old[a] = f0[(size_t)(Q * kC3 + a) * N + n];
+  for (int a = 0; a < kC3; ++a) {
+    old[a] = *src;
+    src += N;
+  }
 #pragma unroll
   for (int a = 0; a < kC3; ++a) {
     double fe;
@@ -575,28 +397,242 @@ __device__ __forceinline__ void collide_dir3(const Ctx3& c, const Fused3& fz,
       else
         val = val + sixth * st.dF[a - 3];
     }
-    dst[a * stride] = val;
+    *dst = val;
+    dst += stride;
   }
 }
 
-// MINB resident blocks of 128 threads per SM bound the registers per thread
-// (4: 128 registers, 3: 168).
-template <int MINB>
-__global__ void __launch_bounds__(128, MINB)
-    k3_collide_node(Ctx3 c, Fused3 fz, const double* __restrict__ f0, double* __restrict__ f1,
-                    double* __restrict__ U, const double* __restrict__ u, int do_repair,
-                    int store_all) {
-  const int N = c.N;
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+// Collision + F repair + push streaming, one thread per node.
+//
+// Bound by memory and by how much of it is in flight: it moves about 1.3 KB per
+// node (f0, f1, U, the swept u, neighbours) at 4.0 TB/s on shell128 (248 us;
+// copying 72 such rows alone reaches 5.3 TB/s with the shifted stores).  What the
+// layout is after:
+//  * little code: the six directions are one loop body, the rows of the axis'
+//    column picked at run time, so the kernel fits the instruction cache.  The
+//    former form, six unrolled directions with the state in registers (271 us,
+//    kept for the wavefront kernel), waited 2.8 of 18 cycles per issue for
+//    instructions, and every material law was compiled into one kernel.
+//  * the node's state (S, P, the changes of P and F: 39 doubles) in shared memory,
+//    a column per thread, so that the loop can index it and the registers hold the
+//    populations in flight.
+//  * the repair's gradient on a straight path when all six neighbours exist.
+//  * L1: 12 warps' worth of staging for all 72 rows (cp.async) left no room in L1
+//    for the lines in flight and for the sectors that neighbouring warps share, and
+//    was slower (377 us); so were more resident blocks, prefetches to L2, one warp
+//    per direction (312 us) and rotating the state through registers (6 to 12 %).
+//
+// MAT >= 0: compiled for that material law.  MINB resident blocks per SM bound the
+// registers per thread.
+constexpr int kCT3 = 128;               // nodes per block
+constexpr int kCState3 = kC3 + 3 * 9;   // S (12), P(F) (9), change of P (9), change of F / 6 (9)
+
+constexpr int kCollideSmem3 = sizeof(double) * kCState3 * kCT3;
+
+template <int MAT, int MINB>
+__global__ void __launch_bounds__(kCT3, MINB)
+    k3_collide(Ctx3 c, Fused3 fz, const double* __restrict__ f0, double* __restrict__ f1,
+                  double* __restrict__ U, const double* __restrict__ u, int do_repair,
+                  int store_all) {
+  extern __shared__ double sm3[];  // [kCState3][kCT3]; every thread uses its own column
+  const int N = c.N, tid = threadIdx.x;
+  const int n = blockIdx.x * kCT3 + tid;
   if (n >= N) return;
-  NodeState3 st;
-  node_prologue3(c, fz, U, u, do_repair, store_all, n, st);
-  collide_dir3<0>(c, fz, st, f0, f1, N, n);
-  collide_dir3<1>(c, fz, st, f0, f1, N, n);
-  collide_dir3<2>(c, fz, st, f0, f1, N, n);
-  collide_dir3<3>(c, fz, st, f0, f1, N, n);
-  collide_dir3<4>(c, fz, st, f0, f1, N, n);
-  collide_dir3<5>(c, fz, st, f0, f1, N, n);
+  const cvlbm3d_problem& p = c.p;
+  const double sixth = 1.0 / 6.0;
+  double* sS = sm3 + tid;
+  double* sP = sS + kC3 * kCT3;
+  double* sdP = sP + 9 * kCT3;
+  double* sdF = sdP + 9 * kCT3;
+  int nb[kQ3];
+#pragma unroll
+  for (int q = 0; q < kQ3; ++q) nb[q] = p.neighbor[(size_t)q * N + n];
+  const int slot = fz.need_slot[n];
+  double S[kC3];
+  {
+    const double* src = U + n;
+#pragma unroll
+    for (int a = 0; a < kC3; ++a) {
+      S[a] = *src;
+      src += N;
+    }
+  }
+  bool repaired = false;
+  {
+    const Mat m = mat3<MAT>(c);
+    const double* F = S + 3;
+    double nn[9];
+    if (do_repair) {
+      // I + grad u of the swept u, as du_axis3: centred with both neighbours, second
+      // order one-sided with two on one side, first order with one, zero with none
+      double* sT = sdF;
+      if ((nb[0] | nb[1] | nb[2] | nb[3] | nb[4] | nb[5]) >= 0) {
+        double num[9];
+        const double* uc = u;
+#pragma unroll
+        for (int comp = 0; comp < 3; ++comp) {
+#pragma unroll
+          for (int ax = 0; ax < 3; ++ax) num[3 * comp + ax] = uc[nb[ax]] - uc[nb[ax + 3]];
+          uc += N;
+        }
+#pragma unroll
+        for (int k = 0; k < 9; ++k) sT[k * kCT3] = divc(num[k], c.h2[k % 3]);
+      } else {
+#pragma unroll 1
+        for (int ax = 0; ax < 3; ++ax) {
+          const int pp = ax == 0 ? nb[0] : ax == 1 ? nb[1] : nb[2];
+          const int pm = ax == 0 ? nb[3] : ax == 1 ? nb[4] : nb[5];
+          const int pp2 = pp >= 0 && pm < 0 ? p.neighbor[(size_t)ax * N + pp] : -1;
+          const int pm2 = pm >= 0 && pp < 0 ? p.neighbor[(size_t)(ax + 3) * N + pm] : -1;
+#pragma unroll 1
+          for (int comp = 0; comp < 3; ++comp) {
+            const double* uc = u + (size_t)comp * N;
+            const double u0 = uc[n];
+            double num = 0.0;
+            bool two = true;  // divided by 2 h (else by h)
+            if (pp >= 0 && pm >= 0) {
+              num = uc[pp] - uc[pm];
+            } else if (pp >= 0) {
+              two = pp2 >= 0;
+              num = two ? -3.0 * u0 + 4.0 * uc[pp] - uc[pp2] : uc[pp] - u0;
+            } else if (pm >= 0) {
+              two = pm2 >= 0;
+              num = two ? 3.0 * u0 - 4.0 * uc[pm] + uc[pm2] : u0 - uc[pm];
+            }
+            sT[(3 * comp + ax) * kCT3] = divc(num, two ? c.h2[ax] : c.h1[ax]);
+          }
+        }
+      }
+      const double beta = fmax(0.0, fmin(1.0, p.blend));
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        const double g = sT[k * kCT3];
+        const double T = k % 4 == 0 ? 1.0 + g : g;
+        nn[k] = F[k] + beta * (T - F[k]);
+      }
+      repaired = det3v(nn) > m.jf;
+    }
+#pragma unroll
+    for (int a = 0; a < kC3; ++a) sS[a * kCT3] = S[a];
+    if (slot >= 0) {
+      double* rowp = fz.Uneed + (size_t)slot * kC3;
+      rowp[0] = S[0];
+      rowp[1] = S[1];
+      rowp[2] = S[2];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) rowp[3 + k] = repaired ? nn[k] : F[k];
+    }
+    if (repaired && store_all) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) U[(size_t)(3 + k) * N + n] = nn[k];
+    }
+    const M3 Po = piola3(F, m);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) sP[k * kCT3] = Po.v[k];
+    if (repaired) {
+      const M3 Pn = piola3(nn, m);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        sdP[k * kCT3] = Pn.v[k] - Po.v[k];
+        sdF[k * kCT3] = sixth * (nn[k] - F[k]);
+      }
+    }
+  }
+  const double k3c = c.k3c, om = p.omega, ff = c.ff;
+  const bool src_v = p.source_mode != kSrcNone, src_f = p.source_mode == kSrcConstant;
+  // the 12 populations of direction q, the F rows in the order of its columns
+  auto load_dir = [&](int q, double* old) {
+    const int ax = q < 3 ? q : q - 3;
+    const int c1 = ax == 2 ? 0 : ax + 1, c2 = ax == 0 ? 2 : ax - 1;
+    const double* src = f0 + (size_t)(q * kC3) * N + n;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      old[a] = *src;
+      src += N;
+    }
+    const size_t o[3] = {(size_t)ax * N, (size_t)c1 * N, (size_t)c2 * N};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) old[3 + 3 * i + j] = src[o[j]];
+      src += 3 * (size_t)N;
+    }
+  };
+  auto push_dir = [&](int q, const double* old) {
+    const int ax = q < 3 ? q : q - 3;
+    const int c1 = ax == 2 ? 0 : ax + 1, c2 = ax == 0 ? 2 : ax - 1;
+    const int col[3] = {ax, c1, c2};  // the axis' own F column first
+    const int nq = q == 0 ? nb[0] : q == 1 ? nb[1] : q == 2 ? nb[2] : q == 3 ? nb[3] : q == 4 ? nb[4] : nb[5];
+    double* d;
+    size_t stride = (size_t)N;
+    if (nq >= 0) {
+      d = f1 + (size_t)(q * kC3) * N + nq;
+    } else {
+      int ell = -1;
+      for (int k = p.node_link_start[n]; k < p.node_link_start[n + 1]; ++k) {
+        const int e = p.node_link_list[k];
+        if (p.link_q[e] == q) ell = e;
+      }
+      if (ell < 0) return;
+      d = fz.scratch + (size_t)ell * kC3;
+      stride = 1;
+    }
+    // velocity rows: flux -P in the axis' column, its sign that of the direction
+    const double s = q < 3 ? 1.0 : -1.0;
+    const double* pP = sP + ax * kCT3;
+    const double* pdP = sdP + ax * kCT3;
+    double vel[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      vel[a] = sS[a * kCT3];
+      const double fe = sixth * (vel[a] + k3c * (s * -pP[3 * a * kCT3]));
+      double val = old[a] + om * (fe - old[a]);
+      if (src_v) val = val + c.sw * source_comp3(a, p.source_mode, p.source, vel);
+      if (repaired) val = val - ff * (s * pdP[3 * a * kCT3]);
+      *d = val;
+      d += stride;
+    }
+    // F rows: flux -v in the axis' column
+    const size_t o[3] = {(size_t)col[0] * stride, (size_t)col[1] * stride, (size_t)col[2] * stride};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const int k = 3 * i + col[j];
+        const double Sa = sS[(3 + k) * kCT3];
+        const double fe = j == 0 ? sixth * (Sa + k3c * (s * -vel[i])) : sixth * Sa;
+        const double v = old[3 + 3 * i + j];
+        double val = v + om * (fe - v);
+        if (src_f) val = val + c.sw * p.source[3 + k];
+        if (repaired) val = val + sdF[k * kCT3];
+        d[o[j]] = val;
+      }
+      d += 3 * stride;
+    }
+  };
+  double va[kC3];
+#pragma unroll 1
+  for (int q = 0; q < kQ3; ++q) {
+    load_dir(q, va);
+    push_dir(q, va);
+  }
+}
+
+using CollideFn3 = void (*)(Ctx3, Fused3, const double*, double*, double*, const double*, int, int);
+
+// The collision compiled for the problem's material law.
+template <int MINB>
+CollideFn3 collide3(int model) {
+  switch (model) {
+    case kMatSVK: return k3_collide<kMatSVK, MINB>;
+    case kMatNeoHooke: return k3_collide<kMatNeoHooke, MINB>;
+    case kMatLogNeoHooke: return k3_collide<kMatLogNeoHooke, MINB>;
+    case kMatMooneyRivlin: return k3_collide<kMatMooneyRivlin, MINB>;
+    case kMatYeoh: return k3_collide<kMatYeoh, MINB>;
+    case kMatGent: return k3_collide<kMatGent, MINB>;
+    case kMatSix: return k3_collide<kMatSix, MINB>;
+    default: return k3_collide<-1, MINB>;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -676,7 +712,7 @@ __global__ void __launch_bounds__(128, MINB)
         if (sweep_due) sweep_node3<true>(c, U, ucol, u, ustar, clock, t_host, n);
       } else {
         NodeState3 st;
-        node_prologue3<true>(c, fz, U, u, do_repair, store_all, n, st);
+        node_prologue3<-1, true>(c, fz, U, u, do_repair, store_all, n, st);
         collide_dir3<0>(c, fz, st, f0, f1, N, n);
         collide_dir3<1>(c, fz, st, f0, f1, N, n);
         collide_dir3<2>(c, fz, st, f0, f1, N, n);

@@ -15,6 +15,12 @@
 
 #define CV_DEV __device__ __forceinline__
 
+#ifdef DIVI
+#define DIVF(a, b) ((a) / (b))
+#endif
+#ifndef DIVF
+#define DIVF div_ieee
+#endif
 namespace cv {
 
 constexpr double kPi = 3.141592653589793238462643383279502884;
@@ -75,9 +81,14 @@ inline DivC make_divc(double b) {
   return d;
 }
 
+// The division itself, out of line: the branches that fall back to it are not
+// taken in a regular run and would only spread the hot code over more instruction
+// cache lines.
+static __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
+
 CV_DEV double divc(double a, const DivC& d) {
   if (mag_hi(a) < d.lim) return quot(a, d.b, d.y, d.e);
-  return a / d.b;
+  return DIVF(a, d.b);
 }
 
 // A divisor formed in the kernel, shared by several numerators of moderate size
@@ -103,7 +114,7 @@ CV_DEV void div_n(const Rcp& r, const double* a, double* out, int n) {
     for (int k = 0; k < n; ++k) out[k] = quot(a[k], r.b, r.y, r.e);
   } else {
 #pragma unroll
-    for (int k = 0; k < n; ++k) out[k] = a[k] / r.b;
+    for (int k = 0; k < n; ++k) out[k] = DIVF(a[k], r.b);
   }
 }
 

@@ -20,7 +20,8 @@ from typing import Literal
 import numpy as np
 
 from .. import _native, _stamp
-from .characteristic_stencil3d import MAX_CHARACTERISTIC_SAMPLES, build_characteristic_weights
+from .characteristic_stencil3d import (MAX_CHARACTERISTIC_SAMPLES, MAX_GRADIENT_SAMPLES,
+                                       MAX_PROBE_SAMPLES, build_characteristic_weights)
 from .geometry3d import (
     BOUNDARY_ID_INNER,
     BOUNDARY_ID_OUTER,
@@ -245,6 +246,23 @@ def _node_link_csr(link_node: np.ndarray, n_nodes: int):
     return start, np.ascontiguousarray(order.astype(np.int32))
 
 
+def _link_major_weights(w):
+    """(link-major characteristic weights, packed) from w [4, 64, links].
+
+    The stencil builder gives the first MAX_GRADIENT_SAMPLES slots gradient weights only
+    and the others value weights only; such tables are packed to [links, 48, 4] (gradient
+    weights, and in slots k < 16 the value weight of slot 48 + k).  Tables of any other
+    form keep [links, 64, 4]."""
+    import torch
+
+    if bool(torch.any(w[0, :MAX_GRADIENT_SAMPLES]) | torch.any(w[1:, MAX_GRADIENT_SAMPLES:])):
+        return w.permute(2, 1, 0).contiguous(), False
+    out = torch.zeros((w.shape[2], MAX_GRADIENT_SAMPLES, 4), dtype=w.dtype, device=w.device)
+    out[:, :, :3] = w[1:, :MAX_GRADIENT_SAMPLES].permute(2, 1, 0)
+    out[:, :MAX_PROBE_SAMPLES, 3] = w[0, MAX_GRADIENT_SAMPLES:].t()
+    return out, True
+
+
 class WarpSparseCurvedBoundaryLBM3D:
     """Active-node sparse curved 3-D solver on sm_100a (reference :3852-4802).
 
@@ -412,6 +430,7 @@ class WarpSparseCurvedBoundaryLBM3D:
         fused = _fused_tables3(tables, geometry.link_q, ck, self.characteristic_stencil,
                                self.n_active)
         self._n_need = 0
+        self._char_packed = False
         if fused is not None:
             need_slot, char_slot, partner, order = fused
             self._n_need = int(need_slot.max()) + 1 if need_slot.size else 0
@@ -421,7 +440,7 @@ class WarpSparseCurvedBoundaryLBM3D:
                 # link-major copies for the fused gather: a link's slots and,
                 # per sample, its four weights side by side
                 t["char_slot_lm"] = t["char_slot"].view(-1, nl).t().contiguous()
-                t["char_w_lm"] = t["char_w"].view(4, -1, nl).permute(2, 1, 0).contiguous()
+                t["char_w_lm"], self._char_packed = _link_major_weights(t["char_w"].view(4, -1, nl))
             t["link_partner"] = dev_i(partner)
             t["link_order"] = dev_i(order)
         link_nodes = np.unique(np.asarray(tables["link_p"], dtype=np.int64))
@@ -490,6 +509,7 @@ class WarpSparseCurvedBoundaryLBM3D:
         for name, tensor in self._tables.items():
             setattr(p, name, _native.ptr(tensor))
         p.n_need = self._n_need
+        p.char_packed = int(self._char_packed)
         p.n_link_nodes = self._n_link_nodes
         p.n_wave_items, p.n_planes = self._n_wave_items, self.nx
         p.overlap = 0  # measured slower on shell192: the link kernels are throughput-bound
@@ -708,8 +728,8 @@ class WarpSparseCurvedBoundaryLBM3D:
             self.time += self.dt
         self.steps += nsteps
 
-    # fused collide kernel: 0 one thread per node (128 registers), 1 six warps
-    # per 32 nodes (shared memory), 2 one thread per node (168 registers)
+    # fused collide kernel: 0 / 1 / 2 four, three or five resident blocks per SM,
+    # 3 / 4 the wavefront form
     NODE_VARIANTS = (0, 1, 2, 3, 4)
 
     @property

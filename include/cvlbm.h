@@ -323,10 +323,9 @@ typedef struct cvlbm3d_problem {
   const int32_t *need_slot;                       /* [n_active] row of U_need holding the
                                                      node's post-step U, or -1 */
   int32_t n_need;                                 /* rows of U_need */
-  int32_t node_variant;                           /* fused collide kernel: 0 one thread per
-                                                     node within 128 registers, 1 six warps
-                                                     per 32 nodes (shared memory), 2 one
-                                                     thread per node within 168 registers,
+  int32_t node_variant;                           /* fused collide kernel: 0 / 1 / 2 four,
+                                                     three or five resident blocks per SM
+                                                     (128, 168, 96 registers per thread),
                                                      3 / 4 the wavefront form (wave_*
                                                      tables) within 128 / 168 registers;
                                                      results are identical */
@@ -359,7 +358,18 @@ typedef struct cvlbm3d_problem {
      four weights as one 4-byte and two 16-byte loads) */
   const int32_t *char_slot_lm;                    /* [n_links][64] = char_slot transposed */
   const double *char_w_lm;                        /* [n_links][64][4]: char_w[k][m][l] at
-                                                     [l][m][k] */
+                                                     [l][m][k]; with char_packed
+                                                     [n_links][48][4] */
+  int32_t char_packed;                            /* nonzero: the value weights vanish in
+                                                     slots 0..47 and the gradient weights in
+                                                     slots 48..63 (as
+                                                     cvlbm3d_build_char_stencil makes them),
+                                                     and char_w_lm holds per link and slot
+                                                     m < 48 the three gradient weights and,
+                                                     for m < 16, the value weight of slot
+                                                     48 + m (else 0): one kernel then does
+                                                     all link work of a step */
+  int32_t reserved0;
 } cvlbm3d_problem;
 
 typedef struct cvlbm3d_fields {
