@@ -599,6 +599,29 @@ int link_priority() {
   return prio;
 }
 
+using LinkFn2 = void (*)(Ctx2, const double*, double*, const double*, const double*, const double*,
+                         double, double, int, const double*, const int32_t*, double*);
+
+LinkFn2 link_kernel2(int model, int recon, int solver) {
+  if (recon == 12) {
+    switch (model) {
+      case kMatNeoHooke:
+        if (solver == kSolverFD) return k_links2g<kMatNeoHooke, 12, kSolverFD>;
+        if (solver == kSolverAcoustic) return k_links2g<kMatNeoHooke, 12, kSolverAcoustic>;
+        if (solver == kSolverEnergy) return k_links2g<kMatNeoHooke, 12, kSolverEnergy>;
+        break;
+      case kMatSVK: return k_links2g<kMatSVK, 12, kSolverFD>;
+      case kMatLogNeoHooke: return k_links2g<kMatLogNeoHooke, 12, kSolverFD>;
+      case kMatMooneyRivlin: return k_links2g<kMatMooneyRivlin, 12, kSolverFD>;
+      case kMatYeoh: return k_links2g<kMatYeoh, 12, kSolverFD>;
+      case kMatGent: return k_links2g<kMatGent, 12, kSolverFD>;
+      case kMatSix: return k_links2g<kMatSix, 12, kSolverFD>;
+      default: break;
+    }
+  }
+  return model == kMatNeoHooke ? k_links2g<kMatNeoHooke> : k_links2g<-1>;
+}
+
 void launch_links(const Ctx2& c, const double* src, double* dst, const double* U,
                   const double* u, const double* clock, double t, double offset,
                   cudaStream_t s, int fused = 0, const double* scratch = nullptr,
@@ -615,19 +638,12 @@ void launch_links(const Ctx2& c, const double* src, double* dst, const double* U
   attr[0].val.priority = link_priority();
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  // builds for the neo-Hooke law with the local_f closure and each Neumann
-  // solver hold only that path's code (fewer instruction-cache misses along
-  // the link's chain); other problems take the generic builds
-  auto kern = k_links2g<-1>;
-  if (c.m.model == kMatNeoHooke) {
-    kern = k_links2g<kMatNeoHooke>;
-    if (c.p.recon == 12 && c.p.normal_solver == kSolverFD)
-      kern = k_links2g<kMatNeoHooke, 12, kSolverFD>;
-    else if (c.p.recon == 12 && c.p.normal_solver == kSolverAcoustic)
-      kern = k_links2g<kMatNeoHooke, 12, kSolverAcoustic>;
-    else if (c.p.recon == 12 && c.p.normal_solver == kSolverEnergy)
-      kern = k_links2g<kMatNeoHooke, 12, kSolverEnergy>;
-  }
+  // builds for one law with the local_f closure and the Neumann solver hold only that
+  // path's code (fewer instruction-cache misses along the link's chain: Mooney-Rivlin
+  // 44 us at 3,824 links in the generic build); the acoustic and energy solvers exist
+  // for the neo-Hooke law only, every other law takes the finite-difference Jacobian.
+  // Problems with another closure take the builds that decide at run time.
+  const auto kern = link_kernel2(c.m.model, c.p.recon, c.p.normal_solver);
   const int tk = link_timer_begin(s);
   cudaLaunchKernelEx(&cfg, kern, c, src, dst, U, u, clock, t, offset, fused, scratch, partner,
                      clock_next);
@@ -687,20 +703,27 @@ struct FusedLaunch2 {
 constexpr int kSplitVariant = 5;
 constexpr int kMaxVariant = 10;
 
-FusedLaunch2 fused_variant(int v) {
+template <int MAT>
+FusedLaunch2 fused_variant_as(int v) {
   switch (v) {
-    case 1: return {k_fused2<8, 2, false>, kTX * 8, fused_smem2<8>(), 8, nullptr};
-    case 2: return {k_fused2<8, 3, false>, kTX * 8, fused_smem2<8>(), 8, nullptr};
-    case 3: return {k_fused2<16, 2, false>, kTX * 16, fused_smem2<16>(), 16, nullptr};
-    case 4: return {k_fused2<4, 4, false>, kTX * 4, fused_smem2<4>(), 4, nullptr};
+    case 1: return {k_fused2<8, 2, false, false, MAT>, kTX * 8, fused_smem2<8>(), 8, nullptr};
+    case 2: return {k_fused2<8, 3, false, false, MAT>, kTX * 8, fused_smem2<8>(), 8, nullptr};
+    case 3: return {k_fused2<16, 2, false, false, MAT>, kTX * 16, fused_smem2<16>(), 16, nullptr};
+    case 4: return {k_fused2<4, 4, false, false, MAT>, kTX * 4, fused_smem2<4>(), 4, nullptr};
     case kSplitVariant: return {nullptr, 0, 0, 16, nullptr};  // split kernels, no tiles used
-    case 6: return {k_fused2<16, 1, true>, kTX * 16, fused_smem2<16>(), 16, k_mom2<16>};
-    case 7: return {k_fused2<8, 3, true>, kTX * 8, fused_smem2<8>(), 8, k_mom2<8>};
-    case 8: return {k_fused2<8, 2, false, true>, kTX * 8, fused_smem2<8, true>(), 8, nullptr};
-    case 9: return {k_fused2<16, 1, false, true>, kTX * 16, fused_smem2<16, true>(), 16, nullptr};
-    case 10: return {k_fused2<4, 4, false, true>, kTX * 4, fused_smem2<4, true>(), 4, nullptr};
-    default: return {k_fused2<16, 1, false>, kTX * 16, fused_smem2<16>(), 16, nullptr};
+    case 6: return {k_fused2<16, 1, true, false, MAT>, kTX * 16, fused_smem2<16>(), 16, k_mom2<16>};
+    case 7: return {k_fused2<8, 3, true, false, MAT>, kTX * 8, fused_smem2<8>(), 8, k_mom2<8>};
+    case 8: return {k_fused2<8, 2, false, true, MAT>, kTX * 8, fused_smem2<8, true>(), 8, nullptr};
+    case 9: return {k_fused2<16, 1, false, true, MAT>, kTX * 16, fused_smem2<16, true>(), 16, nullptr};
+    case 10: return {k_fused2<4, 4, false, true, MAT>, kTX * 4, fused_smem2<4, true>(), 4, nullptr};
+    default: return {k_fused2<16, 1, false, false, MAT>, kTX * 16, fused_smem2<16>(), 16, nullptr};
   }
+}
+
+// The neo-Hooke law gets kernels of its own; the others, with exp and log on the
+// path, share one build.
+FusedLaunch2 fused_variant(int v, int model = -1) {
+  return model == kMatNeoHooke ? fused_variant_as<kMatNeoHooke>(v) : fused_variant_as<-1>(v);
 }
 
 bool fused_ok(const cvlbm2d_problem* p, const cvlbm2d_fields* f) {
@@ -727,7 +750,7 @@ extern "C" int cvlbm2d_run(const cvlbm2d_problem* p, cvlbm2d_fields* f, double t
   k_zero_flag<<<1, 1, 0, s>>>(f->invalid); cv::count_launches(1);
   double t = time0;
   const bool fused = fused_ok(p, f);
-  FusedLaunch2 fl = fused_variant(p->tile_variant);
+  FusedLaunch2 fl = fused_variant(p->tile_variant, p->mat.model);
   const bool split = fused && p->tile_variant == kSplitVariant;
   if (fused && !split)
     cudaFuncSetAttribute(fl.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fl.smem);

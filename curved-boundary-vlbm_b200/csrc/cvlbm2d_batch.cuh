@@ -57,24 +57,36 @@ struct InstState2 {
 
 __device__ __forceinline__ int parity_of(const InstState2& s) { return (int)((s.step - s.base) & 1); }
 
-template <int TY, int MINB>
+template <int TY, int MINB, bool STAGE, int MAT>
 __global__ void __launch_bounds__(kTX * TY, MINB)
     k_batch_nodes2(const Inst2* __restrict__ inst, InstState2* __restrict__ st,
                    const int2* __restrict__ work, int n_work, int store_all) {
   extern __shared__ double smem2[];
+  // The item's instance record in shared memory: one coalesced load instead of a
+  // scattered one for every table pointer and constant the tile needs.  Without the
+  // hoisted halo loads of the single-solver kernel: with the loop around the tile they
+  // spill (8 shells: 55 us per step against 67 with both and 70 before).
+  __shared__ Inst2 sI;
+  __shared__ int s_go;
+  static_assert(sizeof(Inst2) % 8 == 0, "copied in 8-byte words");
   for (int w = blockIdx.x; w < n_work; w += gridDim.x) {
     __syncthreads();  // the previous item's phase C still reads shared memory
     const int2 wk = work[w];
-    if (!st[wk.x].active) continue;
-    const Inst2& I = inst[wk.x];
+    if (threadIdx.x == 0) s_go = st[wk.x].active;
+    for (int t = threadIdx.x; t < (int)(sizeof(Inst2) / 8); t += blockDim.x)
+      reinterpret_cast<unsigned long long*>(&sI)[t] =
+          reinterpret_cast<const unsigned long long*>(inst + wk.x)[t];
+    __syncthreads();
+    if (!s_go) continue;
     const long long step = st[wk.x].step;
     const int par = parity_of(st[wk.x]);
-    const cvlbm2d_problem& p = I.c.p;
+    const cvlbm2d_problem& p = sI.c.p;
     const int sweep = p.disp_interval > 0 && step % p.disp_interval == 0;
     const int repair = p.rep_interval > 0 && step % p.rep_interval == 0;
-    Fused2 fz{nullptr, 0, p.tiles_j, I.need, I.partner, I.scratch, store_all};
-    fused2_tile<TY, false>(I.c, fz, wk.y, I.f[par], I.f[par ^ 1], I.U, I.u, I.us[par], I.us[par ^ 1],
-                    I.invalid, &st[wk.x].clock, 0.0, sweep, repair, smem2);
+    Fused2 fz{nullptr, 0, p.tiles_j, sI.need, sI.partner, sI.scratch, store_all};
+    fused2_tile<TY, false, STAGE, MAT, false>(
+        sI.c, fz, wk.y, sI.f[par], sI.f[par ^ 1], sI.U, sI.u, sI.us[par], sI.us[par ^ 1], sI.invalid,
+        &st[wk.x].clock, 0.0, sweep, repair, smem2);
   }
 }
 
@@ -192,14 +204,26 @@ struct BatchVariant2 {
   int tile_i;
 };
 
-BatchVariant2 batch_variant(int v) {
+template <int MAT>
+BatchVariant2 batch_variant_as(int v) {
   switch (v) {
-    case 1: return {k_batch_nodes2<8, 2>, k_batch_partial2<8>, kTX * 8, fused_smem2<8>(), 8};
-    case 2: return {k_batch_nodes2<8, 3>, k_batch_partial2<8>, kTX * 8, fused_smem2<8>(), 8};
-    case 3: return {k_batch_nodes2<16, 2>, k_batch_partial2<16>, kTX * 16, fused_smem2<16>(), 16};
-    case 4: return {k_batch_nodes2<4, 4>, k_batch_partial2<4>, kTX * 4, fused_smem2<4>(), 4};
-    default: return {k_batch_nodes2<16, 1>, k_batch_partial2<16>, kTX * 16, fused_smem2<16>(), 16};
+    case 1: return {k_batch_nodes2<8, 2, false, MAT>, k_batch_partial2<8>, kTX * 8, fused_smem2<8>(), 8};
+    case 2: return {k_batch_nodes2<8, 3, false, MAT>, k_batch_partial2<8>, kTX * 8, fused_smem2<8>(), 8};
+    case 3: return {k_batch_nodes2<16, 2, false, MAT>, k_batch_partial2<16>, kTX * 16, fused_smem2<16>(), 16};
+    case 4: return {k_batch_nodes2<4, 4, false, MAT>, k_batch_partial2<4>, kTX * 4, fused_smem2<4>(), 4};
+    case 8: return {k_batch_nodes2<8, 2, true, MAT>, k_batch_partial2<8>, kTX * 8, fused_smem2<8, true>(), 8};
+    case 9: return {k_batch_nodes2<16, 1, true, MAT>, k_batch_partial2<16>, kTX * 16, fused_smem2<16, true>(), 16};
+    case 10: return {k_batch_nodes2<4, 4, true, MAT>, k_batch_partial2<4>, kTX * 4, fused_smem2<4, true>(), 4};
+    default: return {k_batch_nodes2<16, 1, false, MAT>, k_batch_partial2<16>, kTX * 16, fused_smem2<16>(), 16};
   }
+}
+
+// Tile variants a batch can run: the plain tiles and the staged ones.
+bool batch_variant_ok(int v) { return (v >= 0 && v <= 4) || (v >= 8 && v <= 10); }
+
+// `neo_hooke`: every instance has that law.
+BatchVariant2 batch_variant(int v, int neo_hooke) {
+  return neo_hooke ? batch_variant_as<kMatNeoHooke>(v) : batch_variant_as<-1>(v);
 }
 
 }  // namespace
@@ -245,7 +269,7 @@ void batch_free(cvlbm2d_batch* b) {
 // Node work items [w0, w1), link items [l0, l1), instances [i0, i1).
 void batch_nodes(cvlbm2d_batch* b, int w0, int w1, int store_all, cudaStream_t s) {
   if (w1 <= w0) return;
-  const BatchVariant2 v = batch_variant(b->variant);
+  const BatchVariant2 v = batch_variant(b->variant, b->all_neo_hooke);
   const int grid = b->node_grid < w1 - w0 ? b->node_grid : w1 - w0;
   v.nodes<<<grid, v.threads, v.smem, s>>>(b->d_inst, b->d_state, b->d_work + w0, w1 - w0,
                                           store_all);
@@ -284,7 +308,7 @@ void batch_step(cvlbm2d_batch* b, int store_all, cudaStream_t s) {
 }
 
 void batch_check(cvlbm2d_batch* b, int check_every, double tol, double t_min, cudaStream_t s) {
-  const BatchVariant2 v = batch_variant(b->variant);
+  const BatchVariant2 v = batch_variant(b->variant, b->all_neo_hooke);
   if (b->n_work <= 0) return;
   v.partial<<<b->node_grid, v.threads, 0, s>>>(b->d_inst, b->d_state, b->d_work, b->n_work,
                                                b->d_partial);
@@ -347,7 +371,7 @@ extern "C" int cvlbm2d_batch_create(int32_t n_inst, const cvlbm2d_problem* probl
     return fail(CVLBM_ERR_INVALID_ARG, "cvlbm2d_batch_create: bad arguments");
   *out = nullptr;
   const int tile_i = cvlbm2d_tile_variant(tile_variant);
-  if (tile_i <= 0 || tile_variant >= kSplitVariant)
+  if (tile_i <= 0 || !batch_variant_ok(tile_variant))
     return fail(CVLBM_ERR_INVALID_ARG, "cvlbm2d_batch_create: unknown tile variant");
   std::vector<Inst2> hi(n_inst);
   std::vector<InstState2> hs(n_inst);
@@ -406,12 +430,6 @@ extern "C" int cvlbm2d_batch_create(int32_t n_inst, const cvlbm2d_problem* probl
   b->variant = tile_variant;
   b->n_work = (int)work.size();
   b->n_lwork = (int)lwork.size();
-  const BatchVariant2 v = batch_variant(tile_variant);
-  cudaFuncSetAttribute(v.nodes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem);
-  int dev = 0, sms = 148, per_sm = 1, per_sm_l = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v.nodes, v.threads, v.smem);
   b->all_neo_hooke = 1;
   b->local_f_solver = problems[0].recon == 12 ? problems[0].normal_solver : -1;
   for (int i = 0; i < n_inst; ++i) {
@@ -419,6 +437,12 @@ extern "C" int cvlbm2d_batch_create(int32_t n_inst, const cvlbm2d_problem* probl
     if (problems[i].recon != 12 || problems[i].normal_solver != b->local_f_solver)
       b->local_f_solver = -1;
   }
+  const BatchVariant2 v = batch_variant(tile_variant, b->all_neo_hooke);
+  cudaFuncSetAttribute(v.nodes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem);
+  int dev = 0, sms = 148, per_sm = 1, per_sm_l = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v.nodes, v.threads, v.smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_l, batch_link_kernel(b), kLinkThreads2,
                                                 0);
   const int full = sms * (per_sm > 0 ? per_sm : 1);

@@ -1,7 +1,15 @@
 // D2Q4x6 step, fused form: one tiled node kernel plus one cooperative link
 // kernel per time step.  Included by cvlbm2d.cu (shares Ctx2 and helpers).
 //
-// Node kernel (k_fused2): a 32x16 tile of nodes per 512-thread block.
+// Node kernel (k_fused2): a tile of 32 x TY nodes per block, compiled for the
+// neo-Hooke law or for all laws.  On small lattices it is one tile's latency (about
+// 15 us cold at 100^2 before, 20 us), beyond that waves of it: so every load of a node
+// is issued at once (active flag, link range and populations are one load level),
+// the first halo node's loads go with the node's own where the registers allow it,
+// nodes with four neighbours take straight-line code in the sweep and the repair, and
+// a population is stored through a pointer and a stride per direction instead of a
+// branch per component.  Per step, launches one by one: 100^2 29 to 25 us, 512^2 51
+// to 40, 701^2 74 to 60 (Mooney-Rivlin 114 to 92), affine 384^2 33 to 25.
 //   A  every node of the tile plus a 3-node halo: moments and collide-time
 //      displacement u from f0, u* into shared memory (halo moments are
 //      recomputed from f0 through L2 instead of being exchanged);
@@ -59,13 +67,17 @@ constexpr size_t fused_smem2() {
          (STAGE ? sizeof(double) * 24 * kTX * TY : 0);
 }
 
+// Shapes that leave 128 registers per thread load the first halo node with the own one.
+template <int TY, int MINB>
+constexpr bool kHoist2 = TY * kTX * MINB <= 512;
+
 // One tile of the fused step (phases A-C above); `tile` is a tile id of the
 // problem's tile list.  Every thread of the block calls it; it returns
 // early only after the last block-wide barrier.  PRE: the collide-time
 // moments of every active node were written by k_mom2 into `mom` this step
 // ([8][N]: U (6), collide-time u (2)), so phase A reads them instead of
 // summing populations (the same doubles: k_mom2 evaluates the same sums).
-template <int TY, bool PRE = false, bool STAGE = false>
+template <int TY, bool PRE = false, bool STAGE = false, int MAT = -1, bool HOIST = false>
 __device__ __forceinline__ void fused2_tile(
     const Ctx2& c, const Fused2& fz, int tile, const double* __restrict__ f0,
     double* __restrict__ f1, double* __restrict__ Ug, double* __restrict__ ug,
@@ -89,52 +101,12 @@ __device__ __forceinline__ void fused2_tile(
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int i = i0 + ty, j = j0 + tx;
   const bool own = i < nx && j < ny;
-  const int n = i * ny + j;
-  const bool own_act = own && p.active[n] != 0;
+  const int n = own ? i * ny + j : 0;
   const int r_own = (ty + kH) * kRX + tx + kH;
-
-  // -- A: region moments -----------------------------------------------------
-  // (loads whose latency would otherwise sit in phase B or C start here)
-  const double time_mid = time_of(clock, t_host, c.hdt);
-  double S[6];
-  double ucol0 = 0.0, ucol1 = 0.0;
-  int own_flag = 0;
-  bool own_need = false;
-  if (own_act) {
-    own_flag = 1 | (p.node_link_start[n + 1] > p.node_link_start[n] ? kFlagLinks : 0);
-    own_need = fz.store_all || fz.need[n];
-    if constexpr (PRE) {
-#pragma unroll
-      for (int a = 0; a < 6; ++a) S[a] = mom[(size_t)a * N + n];
-      ucol0 = mom[6 * (size_t)N + n];
-      ucol1 = mom[7 * (size_t)N + n];
-    } else if constexpr (STAGE) {
-      // moments2c with every population also kept in shared memory
-#pragma unroll
-      for (int a = 0; a < 6; ++a) S[a] = 0.0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int a = 0; a < 6; ++a) {
-          const double v = f0[(q * 6 + a) * N + n];
-          sfo[(q * 6 + a) * kTN + threadIdx.x] = v;
-          S[a] += v;
-        }
-      source_half2(c, S);
-      ucol0 = ustar[n] + c.hdt * S[0];
-      ucol1 = ustar[N + n] + c.hdt * S[1];
-    } else {
-      moments2c(c, f0, n, S);
-      ucol0 = ustar[n] + c.hdt * S[0];
-      ucol1 = ustar[N + n] + c.hdt * S[1];
-    }
-  }
-  // the halo ring only (3 rows above and below the tile, 3 columns either
-  // side of its rows), enumerated so that every lane of a warp takes a halo
-  // node (a loop over the whole region would leave the lanes over interior
-  // nodes idle in most warps)
+  // halo node h of the ring (3 rows above and below the tile, 3 columns either side
+  // of its rows), enumerated so that every lane of a warp takes a halo node
   constexpr int kHalo = 2 * kH * kRX + 2 * kH * kTY;
-  for (int h = threadIdx.x; h < kHalo; h += blockDim.x) {
+  auto halo_node = [&](int h, int& r, int& m) {
     int ri, rj;
     if (h < 2 * kH * kRX) {
       const int hr = h / kRX;  // 0..5: rows 0..2 and TY+3..TY+5
@@ -146,31 +118,120 @@ __device__ __forceinline__ void fused2_tile(
       ri = kH + row;
       rj = col < kH ? col : kTX + col;
     }
-    const int r = ri * kRX + rj;
+    r = ri * kRX + rj;
     const int gi = i0 - kH + ri, gj = j0 - kH + rj;
-    const bool inb = gi >= 0 && gi < nx && gj >= 0 && gj < ny;
-    const int m = gi * ny + gj;
-    const int act = inb ? p.active[m] : 0;
-    sA[r] = act ? 1 | (p.node_link_start[m + 1] > p.node_link_start[m] ? kFlagLinks : 0) : 0;
-    if (act) {
-      if constexpr (PRE) {
+    m = gi * ny + gj;
+    return gi >= 0 && gi < nx && gj >= 0 && gj < ny;
+  };
+  auto sum24 = [&](const double* v, double* S) {  // reference order: for q: for a
 #pragma unroll
-        for (int k = 0; k < 4; ++k) sF[k][r] = mom[(size_t)(2 + k) * N + m];
-        sU[0][r] = mom[6 * (size_t)N + m];
-        sU[1][r] = mom[7 * (size_t)N + m];
-      } else {
-        double Sh[6];
-        moments2c(c, f0, m, Sh);
-        sF[0][r] = Sh[2];
-        sF[1][r] = Sh[3];
-        sF[2][r] = Sh[4];
-        sF[3][r] = Sh[5];
-        sU[0][r] = ustar[m] + c.hdt * Sh[0];
-        sU[1][r] = ustar[N + m] + c.hdt * Sh[1];
+    for (int a = 0; a < 6; ++a) S[a] = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int a = 0; a < 6; ++a) S[a] += v[q * 6 + a];
+    source_half2(c, S);
+  };
+  auto put_halo = [&](int r, int flag, const double* S, double us0, double us1) {
+    sA[r] = flag;
+    sF[0][r] = flag ? S[2] : 0.0;
+    sF[1][r] = flag ? S[3] : 0.0;
+    sF[2][r] = flag ? S[4] : 0.0;
+    sF[3][r] = flag ? S[5] : 0.0;
+    sU[0][r] = flag ? us0 + c.hdt * S[0] : 0.0;
+    sU[1][r] = flag ? us1 + c.hdt * S[1] : 0.0;
+  };
+
+  // -- A: region moments -----------------------------------------------------
+  // Every load of a node is issued at once, whether the node turns out to be active
+  // or not (its populations exist all the same), so that the active flag, the link
+  // range and the populations are one load level instead of two.
+  const double time_mid = time_of(clock, t_host, c.hdt);
+  double S[6];
+  double ucol0 = 0.0, ucol1 = 0.0;
+  int own_flag = 0, own_act_i = 0;
+  bool own_need = false;
+  int h_first = threadIdx.x;  // first halo node of the loop below
+  if constexpr (PRE) {
+    own_act_i = own ? p.active[n] : 0;
+    if (own_act_i) {
+      own_flag = 1 | (p.node_link_start[n + 1] > p.node_link_start[n] ? kFlagLinks : 0);
+      own_need = fz.store_all || fz.need[n];
+#pragma unroll
+      for (int a = 0; a < 6; ++a) S[a] = mom[(size_t)a * N + n];
+      ucol0 = mom[6 * (size_t)N + n];
+      ucol1 = mom[7 * (size_t)N + n];
+    }
+  } else {
+    double v[24], us0 = 0.0, us1 = 0.0;
+    int l0 = 0, l1 = 0;
+    if (own) {
+      own_act_i = p.active[n];
+#pragma unroll
+      for (int k = 0; k < 24; ++k) v[k] = f0[k * N + n];
+      us0 = ustar[n];
+      us1 = ustar[N + n];
+      l0 = p.node_link_start[n];
+      l1 = p.node_link_start[n + 1];
+      own_need = fz.need[n] != 0;
+    }
+    if constexpr (HOIST) {
+      // the thread's first halo node, its loads in flight with the node's own
+      double hv[24], hu0 = 0.0, hu1 = 0.0;
+      int r = -1, m = 0, ha = 0, k0 = 0, k1 = 0;
+      if (h_first < kHalo && halo_node(h_first, r, m)) {
+        ha = p.active[m];
+#pragma unroll
+        for (int k = 0; k < 24; ++k) hv[k] = f0[k * N + m];
+        hu0 = ustar[m];
+        hu1 = ustar[N + m];
+        k0 = p.node_link_start[m];
+        k1 = p.node_link_start[m + 1];
       }
+      if (r >= 0) {
+        double Sh[6];
+        if (ha) sum24(hv, Sh);
+        put_halo(r, ha ? 1 | (k1 > k0 ? kFlagLinks : 0) : 0, Sh, hu0, hu1);
+      }
+      h_first += blockDim.x;
+    }
+    if (own_act_i) {
+      own_flag = 1 | (l1 > l0 ? kFlagLinks : 0);
+      own_need = own_need || fz.store_all;
+      if constexpr (STAGE) {
+#pragma unroll
+        for (int k = 0; k < 24; ++k) sfo[k * kTN + threadIdx.x] = v[k];
+      }
+      sum24(v, S);
+      ucol0 = us0 + c.hdt * S[0];
+      ucol1 = us1 + c.hdt * S[1];
+    }
+  }
+  const bool own_act = own_act_i != 0;
+  for (int h = h_first; h < kHalo; h += blockDim.x) {
+    int r, m;
+    const bool inb = halo_node(h, r, m);
+    if constexpr (PRE) {
+      const int act = inb ? p.active[m] : 0;
+      sA[r] = act ? 1 | (p.node_link_start[m + 1] > p.node_link_start[m] ? kFlagLinks : 0) : 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) sF[k][r] = act ? mom[(size_t)(2 + k) * N + m] : 0.0;
+      sU[0][r] = act ? mom[6 * (size_t)N + m] : 0.0;
+      sU[1][r] = act ? mom[7 * (size_t)N + m] : 0.0;
     } else {
-      sF[0][r] = sF[1][r] = sF[2][r] = sF[3][r] = 0.0;
-      sU[0][r] = sU[1][r] = 0.0;
+      double hv[24], Sh[6], hu0 = 0.0, hu1 = 0.0;
+      int ha = 0, k0 = 0, k1 = 0;
+      if (inb) {
+        ha = p.active[m];
+#pragma unroll
+        for (int k = 0; k < 24; ++k) hv[k] = f0[k * N + m];
+        hu0 = ustar[m];
+        hu1 = ustar[N + m];
+        k0 = p.node_link_start[m];
+        k1 = p.node_link_start[m + 1];
+      }
+      if (ha) sum24(hv, Sh);
+      put_halo(r, ha ? 1 | (k1 > k0 ? kFlagLinks : 0) : 0, Sh, hu0, hu1);
     }
   }
   sA[r_own] = own_flag;
@@ -199,6 +260,23 @@ __device__ __forceinline__ void fused2_tile(
     if (!do_sweep) {
       sN[0][s] = sU[0][r];
       sN[1][s] = sU[1][r];
+      continue;
+    }
+    const double hx = 0.5 * p.dx, hy = 0.5 * p.dy;
+    if (sA[r] == 1 && sA[r + kRX] && sA[r - kRX] && sA[r + 1] && sA[r - 1]) {
+      // no cut link: the sums of the general case below with a weight sum of 4
+      const double f0 = sF[0][r] - 1.0, f1_ = sF[1][r], f2 = sF[2][r], f3 = sF[3][r] - 1.0;
+      const int xp = r + kRX, xm = r - kRX, yp = r + 1, ym = r - 1;
+      const double rx = ((sU[0][xp] - hx * (f0 + (sF[0][xp] - 1.0))) +
+                         (sU[0][xm] + hx * ((sF[0][xm] - 1.0) + f0))) +
+                        (sU[0][yp] - hy * (f1_ + sF[1][yp]));
+      const double ry = ((sU[1][xp] - hx * (f2 + sF[2][xp])) + (sU[1][xm] + hx * (sF[2][xm] + f2))) +
+                        (sU[1][yp] - hy * (f3 + (sF[3][yp] - 1.0)));
+      const double sx = rx + (sU[0][ym] + hy * (sF[1][ym] + f1_));
+      const double sy = ry + (sU[1][ym] + hy * ((sF[3][ym] - 1.0) + f3));
+      const double u0 = sU[0][r], u1 = sU[1][r];
+      sN[0][s] = u0 + p.relax * (sx * 0.25 - u0);
+      sN[1][s] = u1 + p.relax * (sy * 0.25 - u1);
       continue;
     }
     const int gi = i0 - 2 + si, gj = j0 - 2 + sj;
@@ -237,7 +315,6 @@ __device__ __forceinline__ void fused2_tile(
       rx = rx + w2 * tx_;
       ry = ry + w2 * ty_;
     }
-    const double hx = 0.5 * p.dx, hy = 0.5 * p.dy;
     if (sA[r + kRX]) {  // +x (i+1)
       const int o = r + kRX;
       rx += sU[0][o] - hx * ((sF[0][r] - 1.0) + (sF[0][o] - 1.0));
@@ -276,7 +353,8 @@ __device__ __forceinline__ void fused2_tile(
   // -- C: repair, collision, streaming (owner) -------------------------------
   const int s_own = (ty + 2) * kSX + tx + 2;
   const double un0 = sN[0][s_own], un1 = sN[1][s_own];
-  const Mat& m = c.m;
+  Mat m = c.m;
+  if (MAT >= 0) m.model = MAT;
   double Fn[4] = {S[2], S[3], S[4], S[5]};
   bool repaired = false;
   if (do_repair) {
@@ -289,6 +367,14 @@ __device__ __forceinline__ void fused2_tile(
       // one-sided / centred derivatives of the swept displacement
       // (two_d/curved_boundary_warp.py:3213-3272) on the shared tile+2 window
       double g[2][2];
+      if (sA[r_own - kRX] && sA[r_own + kRX] && sA[r_own - 1] && sA[r_own + 1]) {
+#pragma unroll
+        for (int comp = 0; comp < 2; ++comp) {
+          const double* w = sN[comp];
+          g[comp][0] = divc(w[s_own + kSX] - w[s_own - kSX], c.dx2);
+          g[comp][1] = divc(w[s_own + 1] - w[s_own - 1], c.dy2);
+        }
+      } else {
 #pragma unroll
       for (int ax = 0; ax < 2; ++ax) {
         const int rs = ax == 0 ? kRX : 1, ss = ax == 0 ? kSX : 1;
@@ -317,6 +403,7 @@ __device__ __forceinline__ void fused2_tile(
           }
           g[comp][ax] = d;
         }
+      }
       }
       const double t11 = 1.0 + g[0][0], t12 = g[0][1], t21 = g[1][0], t22 = 1.0 + g[1][1];
       double alpha = fmax(0.0, fmin(1.0, p.blend));
@@ -348,21 +435,27 @@ __device__ __forceinline__ void fused2_tile(
     const P2 Pn = piola2(Fn[0], Fn[1], Fn[2], Fn[3], m);
     dP = {Pn.a - Po.a, Pn.b - Po.b, Pn.c - Po.c, Pn.d - Po.d};
   }
-  // destinations of the four directions: a neighbour node, a cut link's
-  // scratch row, or nowhere (a cut link without scratch)
-  int dst[4];
+  // destinations of the four directions: the row of a neighbour node in f1 (stride N)
+  // or of a cut link in the scratch (stride 1); neither: a cut link without scratch
+  double* dst[4];
+  int stride[4];
+  bool out[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int cq = cx2(q), cy = cy2(q);
+    out[q] = true;
     if (sA[r_own + cq * kRX + cy] != 0) {
-      dst[q] = n + cq * ny + cy;
+      dst[q] = f1 + (q * 6 * N + n + cq * ny + cy);
+      stride[q] = N;
     } else {
       int ell_out = -1;
       for (int k = p.node_link_start[n]; k < p.node_link_start[n + 1]; ++k) {
         const int e = p.node_link_list[k];
         if (p.link_q[e] == q) ell_out = e;
       }
-      dst[q] = ell_out >= 0 ? -2 - ell_out : -1;
+      out[q] = ell_out >= 0;
+      dst[q] = fz.scratch + (size_t)(ell_out >= 0 ? ell_out : 0) * 6;
+      stride[q] = 1;
     }
   }
   const bool add_src = p.source_mode != kSrcNone;
@@ -407,11 +500,7 @@ __device__ __forceinline__ void fused2_tile(
           v = v + rF;
         }
       }
-      const int d = dst[q];
-      if (d >= 0)
-        f1[(q * 6 + a) * N + d] = v;
-      else if (d <= -2)
-        fz.scratch[(size_t)(-2 - d) * 6 + a] = v;
+      if (out[q]) dst[q][a * stride[q]] = v;
     }
   }
   const double dt = p.dt;
@@ -433,7 +522,7 @@ __device__ __forceinline__ void fused2_tile(
 
 // Tile kTX x TY, one node per thread; MINB resident blocks per SM bounds the
 // registers per thread (tuned per problem, see curved_lbm autotune).
-template <int TY, int MINB, bool PRE, bool STAGE = false>
+template <int TY, int MINB, bool PRE, bool STAGE, int MAT>
 __global__ void __launch_bounds__(kTX * TY, MINB)
     k_fused2(Ctx2 c, Fused2 fz, const double* __restrict__ f0, double* __restrict__ f1,
              double* __restrict__ Ug, double* __restrict__ ug,
@@ -441,7 +530,7 @@ __global__ void __launch_bounds__(kTX * TY, MINB)
              int* __restrict__ invalid, const double* clock, double t_host, int do_sweep,
              int do_repair, const double* __restrict__ mom) {
   extern __shared__ double smem2[];
-  fused2_tile<TY, PRE, STAGE>(c, fz, fz.tiles[blockIdx.x], f0, f1, Ug, ug, ustar, ustar_out,
+  fused2_tile<TY, PRE, STAGE, MAT, kHoist2<TY, MINB>>(c, fz, fz.tiles[blockIdx.x], f0, f1, Ug, ug, ustar, ustar_out,
                               invalid, clock, t_host, do_sweep, do_repair, smem2, mom);
 }
 
