@@ -681,42 +681,38 @@ Overlap2* overlap_resources(cudaStream_t s) {
 }
 
 using FusedFn2 = void (*)(Ctx2, Fused2, const double*, double*, double*, double*, const double*,
-                          double*, int*, const double*, double, int, int, const double*);
-using MomFn2 = void (*)(Ctx2, Fused2, const double*, const double*, double*);
-
+                          double*, int*, const double*, double, int, int);
 struct FusedLaunch2 {
   FusedFn2 fn;
   int threads;
   size_t smem;
   int tile_i;
-  MomFn2 mom;  // PRE form: moments kernel launched before the tile kernel, else null
 };
 
-// Compiled tile variants: (tile rows, resident blocks per SM, PRE).  The tile
-// list in the problem must have been built for the variant's tile height.
-// Variant 5 selects the split form (cvlbm2d_split.cuh) instead of a tile
-// shape; variants 6 and 7 are the PRE form (moments of every active node
-// written once per step by k_mom2 into fields->fpost, halo moments read from
-// there instead of recomputed), which runs without the link overlap;
-// variants 8-10 keep the owned nodes' populations in shared memory from the
-// moments to the collision (STAGE) instead of reloading them.
+// Compiled tile variants: tile rows, resident blocks per SM, STAGE.  The tile list in
+// the problem must have been built for the variant's tile height.  Variant 5 selects
+// the split form (cvlbm2d_split.cuh) instead of a tile shape; variants 7 to 10 keep the
+// owned nodes' populations in shared memory from the moments to the collision (STAGE)
+// instead of reloading them.  The heights differ because the tiles of a lattice fill
+// whole waves of (SMs x resident blocks) badly or well: 512^2 is 608 tiles of 8 rows,
+// 2.05 waves of 296, but 1.7 of 10 rows (35.9 and 33.9 us per step).
 constexpr int kSplitVariant = 5;
 constexpr int kMaxVariant = 10;
 
 template <int MAT>
 FusedLaunch2 fused_variant_as(int v) {
   switch (v) {
-    case 1: return {k_fused2<8, 2, false, false, MAT>, kTX * 8, fused_smem2<8>(), 8, nullptr};
-    case 2: return {k_fused2<8, 3, false, false, MAT>, kTX * 8, fused_smem2<8>(), 8, nullptr};
-    case 3: return {k_fused2<16, 2, false, false, MAT>, kTX * 16, fused_smem2<16>(), 16, nullptr};
-    case 4: return {k_fused2<4, 4, false, false, MAT>, kTX * 4, fused_smem2<4>(), 4, nullptr};
-    case kSplitVariant: return {nullptr, 0, 0, 16, nullptr};  // split kernels, no tiles used
-    case 6: return {k_fused2<16, 1, true, false, MAT>, kTX * 16, fused_smem2<16>(), 16, k_mom2<16>};
-    case 7: return {k_fused2<8, 3, true, false, MAT>, kTX * 8, fused_smem2<8>(), 8, k_mom2<8>};
-    case 8: return {k_fused2<8, 2, false, true, MAT>, kTX * 8, fused_smem2<8, true>(), 8, nullptr};
-    case 9: return {k_fused2<16, 1, false, true, MAT>, kTX * 16, fused_smem2<16, true>(), 16, nullptr};
-    case 10: return {k_fused2<4, 4, false, true, MAT>, kTX * 4, fused_smem2<4, true>(), 4, nullptr};
-    default: return {k_fused2<16, 1, false, false, MAT>, kTX * 16, fused_smem2<16>(), 16, nullptr};
+    case 1: return {k_fused2<8, 2, false, MAT>, kTX * 8, fused_smem2<8>(), 8};
+    case 2: return {k_fused2<8, 3, false, MAT>, kTX * 8, fused_smem2<8>(), 8};
+    case 3: return {k_fused2<16, 2, false, MAT>, kTX * 16, fused_smem2<16>(), 16};
+    case 4: return {k_fused2<4, 4, false, MAT>, kTX * 4, fused_smem2<4>(), 4};
+    case kSplitVariant: return {nullptr, 0, 0, 16};  // split kernels, no tiles used
+    case 6: return {k_fused2<10, 2, false, MAT>, kTX * 10, fused_smem2<10>(), 10};
+    case 7: return {k_fused2<9, 2, true, MAT>, kTX * 9, fused_smem2<9, true>(), 9};
+    case 8: return {k_fused2<8, 2, true, MAT>, kTX * 8, fused_smem2<8, true>(), 8};
+    case 9: return {k_fused2<16, 1, true, MAT>, kTX * 16, fused_smem2<16, true>(), 16};
+    case 10: return {k_fused2<4, 4, true, MAT>, kTX * 4, fused_smem2<4, true>(), 4};
+    default: return {k_fused2<16, 1, false, MAT>, kTX * 16, fused_smem2<16>(), 16};
   }
 }
 
@@ -729,7 +725,7 @@ FusedLaunch2 fused_variant(int v, int model = -1) {
 bool fused_ok(const cvlbm2d_problem* p, const cvlbm2d_fields* f) {
   const FusedLaunch2 fl = fused_variant(p->tile_variant);
   return p->tiles && p->need_fields && p->link_partner && f->link_scratch && p->lsq_node &&
-         p->disp_sweeps <= 1 && fl.tile_i == p->tile_i && (!fl.mom || f->fpost) &&
+         p->disp_sweeps <= 1 && fl.tile_i == p->tile_i &&
          p->collision_model == 0 && !(p->kinetic_filter > 0.0) &&
          // the fused node kernel indexes populations with 32-bit offsets
          24LL * p->nx * p->ny < 2147483647LL;
@@ -759,7 +755,7 @@ extern "C" int cvlbm2d_run(const cvlbm2d_problem* p, cvlbm2d_fields* f, double t
   double* us_cur = f->u_star;
   double* us_nxt = f->u_next;
   Overlap2* ov = nullptr;
-  if (fused && !split && !fl.mom && p->overlap && p->n_tiles_inner > 0 &&
+  if (fused && !split && p->overlap && p->n_tiles_inner > 0 &&
       p->n_tiles_inner < p->n_tiles && nsteps > 0) {
     ov = overlap_resources(s);
     if (ov) {
@@ -805,13 +801,12 @@ extern "C" int cvlbm2d_run(const cvlbm2d_problem* p, cvlbm2d_fields* f, double t
         cudaStreamWaitEvent(ov->inner, ov->boundary_done, 0);
       }
       fl.fn<<<n_bd, fl.threads, fl.smem, s>>>(c, fz_bd, f->f0, f->f1, f->U, f->u, us_cur,
-                                              us_nxt, f->invalid, clock, t, sweep, repair,
-                                              nullptr);
+                                              us_nxt, f->invalid, clock, t, sweep, repair);
       cudaEventRecord(ov->boundary_done, s);
       // inner tiles read no time (they have no cut-point anchors)
       fl.fn<<<n_in, fl.threads, fl.smem, ov->inner>>>(c, fz_in, f->f0, f->f1, f->U, f->u, us_cur,
                                                       us_nxt, f->invalid, nullptr, t, sweep,
-                                                      repair, nullptr);
+                                                      repair);
       cudaEventRecord(ov->inner_done, ov->inner);
       cv::count_launches(2);
       double* us = us_cur;
@@ -824,13 +819,8 @@ extern "C" int cvlbm2d_run(const cvlbm2d_problem* p, cvlbm2d_fields* f, double t
                 f->link_scratch, k == nsteps - 1};
       int tk = timer_begin(s);
       if (p->n_tiles > 0) {
-        if (fl.mom) {
-          fl.mom<<<p->n_tiles, fl.threads, 0, s>>>(c, fz, f->f0, us_cur, f->fpost);
-          cv::count_launches(1);
-        }
         fl.fn<<<p->n_tiles, fl.threads, fl.smem, s>>>(c, fz, f->f0, f->f1, f->U, f->u, us_cur,
-                                                      us_nxt, f->invalid, clock, t, sweep, repair,
-                                                      f->fpost);
+                                                      us_nxt, f->invalid, clock, t, sweep, repair);
         cv::count_launches(1);
       }
       double* us = us_cur;

@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kTX * TY, MINB)
     const int sweep = p.disp_interval > 0 && step % p.disp_interval == 0;
     const int repair = p.rep_interval > 0 && step % p.rep_interval == 0;
     Fused2 fz{nullptr, 0, p.tiles_j, sI.need, sI.partner, sI.scratch, store_all};
-    fused2_tile<TY, false, STAGE, MAT, false>(
+    fused2_tile<TY, STAGE, MAT, false>(
         sI.c, fz, wk.y, sI.f[par], sI.f[par ^ 1], sI.U, sI.u, sI.us[par], sI.us[par ^ 1], sI.invalid,
         &st[wk.x].clock, 0.0, sweep, repair, smem2);
   }
@@ -218,7 +218,7 @@ BatchVariant2 batch_variant_as(int v) {
   }
 }
 
-// Tile variants a batch can run: the plain tiles and the staged ones.
+// Tile variants a batch can run: the residual reduction wants a power of two threads.
 bool batch_variant_ok(int v) { return (v >= 0 && v <= 4) || (v >= 8 && v <= 10); }
 
 // `neo_hooke`: every instance has that law.

@@ -73,17 +73,13 @@ constexpr bool kHoist2 = TY * kTX * MINB <= 512;
 
 // One tile of the fused step (phases A-C above); `tile` is a tile id of the
 // problem's tile list.  Every thread of the block calls it; it returns
-// early only after the last block-wide barrier.  PRE: the collide-time
-// moments of every active node were written by k_mom2 into `mom` this step
-// ([8][N]: U (6), collide-time u (2)), so phase A reads them instead of
-// summing populations (the same doubles: k_mom2 evaluates the same sums).
-template <int TY, bool PRE = false, bool STAGE = false, int MAT = -1, bool HOIST = false>
+// early only after the last block-wide barrier.
+template <int TY, bool STAGE = false, int MAT = -1, bool HOIST = false>
 __device__ __forceinline__ void fused2_tile(
     const Ctx2& c, const Fused2& fz, int tile, const double* __restrict__ f0,
     double* __restrict__ f1, double* __restrict__ Ug, double* __restrict__ ug,
     const double* __restrict__ ustar, double* __restrict__ ustar_out, int* __restrict__ invalid,
-    const double* clock, double t_host, int do_sweep, int do_repair, double* smem2,
-    const double* __restrict__ mom = nullptr) {
+    const double* clock, double t_host, int do_sweep, int do_repair, double* smem2) {
   constexpr int kTY = TY;
   constexpr int kRN = kRX * (TY + 2 * kH);
   constexpr int kSN = kSX * (TY + 4);
@@ -152,17 +148,7 @@ __device__ __forceinline__ void fused2_tile(
   int own_flag = 0, own_act_i = 0;
   bool own_need = false;
   int h_first = threadIdx.x;  // first halo node of the loop below
-  if constexpr (PRE) {
-    own_act_i = own ? p.active[n] : 0;
-    if (own_act_i) {
-      own_flag = 1 | (p.node_link_start[n + 1] > p.node_link_start[n] ? kFlagLinks : 0);
-      own_need = fz.store_all || fz.need[n];
-#pragma unroll
-      for (int a = 0; a < 6; ++a) S[a] = mom[(size_t)a * N + n];
-      ucol0 = mom[6 * (size_t)N + n];
-      ucol1 = mom[7 * (size_t)N + n];
-    }
-  } else {
+  {
     double v[24], us0 = 0.0, us1 = 0.0;
     int l0 = 0, l1 = 0;
     if (own) {
@@ -211,14 +197,7 @@ __device__ __forceinline__ void fused2_tile(
   for (int h = h_first; h < kHalo; h += blockDim.x) {
     int r, m;
     const bool inb = halo_node(h, r, m);
-    if constexpr (PRE) {
-      const int act = inb ? p.active[m] : 0;
-      sA[r] = act ? 1 | (p.node_link_start[m + 1] > p.node_link_start[m] ? kFlagLinks : 0) : 0;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) sF[k][r] = act ? mom[(size_t)(2 + k) * N + m] : 0.0;
-      sU[0][r] = act ? mom[6 * (size_t)N + m] : 0.0;
-      sU[1][r] = act ? mom[7 * (size_t)N + m] : 0.0;
-    } else {
+    {
       double hv[24], Sh[6], hu0 = 0.0, hu1 = 0.0;
       int ha = 0, k0 = 0, k1 = 0;
       if (inb) {
@@ -522,39 +501,16 @@ __device__ __forceinline__ void fused2_tile(
 
 // Tile kTX x TY, one node per thread; MINB resident blocks per SM bounds the
 // registers per thread (tuned per problem, see curved_lbm autotune).
-template <int TY, int MINB, bool PRE, bool STAGE, int MAT>
+template <int TY, int MINB, bool STAGE, int MAT>
 __global__ void __launch_bounds__(kTX * TY, MINB)
     k_fused2(Ctx2 c, Fused2 fz, const double* __restrict__ f0, double* __restrict__ f1,
              double* __restrict__ Ug, double* __restrict__ ug,
              const double* __restrict__ ustar, double* __restrict__ ustar_out,
              int* __restrict__ invalid, const double* clock, double t_host, int do_sweep,
-             int do_repair, const double* __restrict__ mom) {
+             int do_repair) {
   extern __shared__ double smem2[];
-  fused2_tile<TY, PRE, STAGE, MAT, kHoist2<TY, MINB>>(c, fz, fz.tiles[blockIdx.x], f0, f1, Ug, ug, ustar, ustar_out,
-                              invalid, clock, t_host, do_sweep, do_repair, smem2, mom);
-}
-
-// Collide-time moments of the active nodes of the listed tiles, for the PRE
-// form of the tile kernel: mom[0..5] = U with the damping half step
-// (moments2), mom[6..7] = u* + dt/2 v.  One thread per node, coalesced rows.
-template <int TY>
-__global__ void __launch_bounds__(kTX * TY)
-    k_mom2(Ctx2 c, Fused2 fz, const double* __restrict__ f0, const double* __restrict__ ustar,
-           double* __restrict__ mom) {
-  const cvlbm2d_problem& p = c.p;
-  const int N = c.N;
-  const int tile = fz.tiles[blockIdx.x];
-  const int i = (tile / fz.tiles_j) * TY + (threadIdx.x >> 5);
-  const int j = (tile % fz.tiles_j) * kTX + (threadIdx.x & 31);
-  if (i >= p.nx || j >= p.ny) return;
-  const int n = i * p.ny + j;
-  if (p.active[n] == 0) return;
-  double S[6];
-  moments2c(c, f0, n, S);
-#pragma unroll
-  for (int a = 0; a < 6; ++a) mom[(size_t)a * N + n] = S[a];
-  mom[6 * (size_t)N + n] = ustar[n] + 0.5 * p.dt * S[0];
-  mom[7 * (size_t)N + n] = ustar[N + n] + 0.5 * p.dt * S[1];
+  fused2_tile<TY, STAGE, MAT, kHoist2<TY, MINB>>(c, fz, fz.tiles[blockIdx.x], f0, f1, Ug, ug, ustar, ustar_out,
+                              invalid, clock, t_host, do_sweep, do_repair, smem2);
 }
 
 // ---------------------------------------------------------------------------

@@ -61,7 +61,7 @@ class BatchedCurvedBoundaryLBM2D:
             # the solvers' shape if it was chosen for them, else the staged 8 x 32 tile
             # (24 shells: 223 us per step against 253 with the solvers' default)
             tile_variant = self.solvers[0].tile_variant
-            if tile_variant == DEFAULT_TILE_VARIANT or tile_variant not in BATCH_VARIANTS:
+            if tile_variant == DEFAULT_TILE_VARIANT or int(tile_variant) not in BATCH_VARIANTS:
                 tile_variant = BATCH_DEFAULT_VARIANT
         self.tile_variant = int(tile_variant)
         self.handle = None

@@ -217,10 +217,13 @@ class CurvedBoundarySpec:
 
 
 TILE_J = 32
-# tile shape before any autotune(): 8 x 32 nodes, two blocks per SM.  From 64^2 to 701^2
-# it is within 3 % of the best shape (512^2: 35.7 us per step, 701^2: 56.8; the 16-row
-# tile with one block per SM 36.7 and 57.6); autotune() picks per problem.
+# Tile shapes before any autotune(): 8 x 32 nodes, two blocks per SM, while those tiles
+# fit one wave; beyond that 10 x 32 (also two blocks), which wastes less of the last
+# wave and of the halo (384^2: 28.6 us per step against 25.4, 512^2: 35.9 / 33.9, 701^2
+# Mooney-Rivlin: 76.0 / 68.6; 200^2, one wave: 20.9 / 22.0).
 DEFAULT_TILE_VARIANT = 1
+DEFAULT_TILE_VARIANT_LARGE = 6
+DEFAULT_TILES_PER_SM = 2
 
 
 def _tile_list(active: np.ndarray, tile_i: int):
@@ -534,6 +537,9 @@ class WarpCurvedBoundaryLBM2D:
         self.use_graphs = True
         self._problem = self._make_problem()
         self._select_variant(self.tile_variant)
+        sms = torch.cuda.get_device_properties(self._tdev).multi_processor_count
+        if self._problem.n_tiles > DEFAULT_TILES_PER_SM * sms:
+            self._select_variant(DEFAULT_TILE_VARIANT_LARGE)
         self.initialize_identity(init_order=1)
 
     # -- native plumbing ---------------------------------------------------
