@@ -668,12 +668,11 @@ extern "C" int cvlbm3d_run(const cvlbm3d_problem* p, cvlbm3d_fields* f, double t
     const bool wave = wave_ok3(p, f) && N > 0;
     const bool packed = p->char_packed && p->char_slot_lm && p->char_w_lm;
     const LinkFn3 link_fn = link_finish3(c.m.model);
-    const CollideFn3 collide_fn = p->node_variant == 1   ? collide3<3>(c.m.model)
-                                  : p->node_variant == 2 ? collide3<5>(c.m.model)
-                                                         : collide3<4>(c.m.model);
-    if (kCollideSmem3 > 48 * 1024)
-      cudaFuncSetAttribute(collide_fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)kCollideSmem3);
+    static_assert(kCollideSmem3 <= 48 * 1024, "no opt-in needed");
+    const CollideFn3 collide_fn = p->node_variant == 1   ? collide3<3, false>(c.m.model)
+                                  : p->node_variant == 2 ? collide3<5, false>(c.m.model)
+                                                         : collide3<4, false>(c.m.model);
+    const CollideFn3 collide_mom = collide3<4, true>(c.m.model);
     Overlap3* ov = nullptr;
     if (!wave && p->overlap && p->disp_interval == 1 && N > 0 && L > 0 && p->link_nodes &&
         p->n_link_nodes > 0 && nsteps > 1)
@@ -684,6 +683,7 @@ extern "C" int cvlbm3d_run(const cvlbm3d_problem* p, cvlbm3d_fields* f, double t
       const long long step = step0 + k;
       const int sweep = N > 0 && due(p->disp_interval, step);
       const int repair = due(p->rep_interval, step);
+      const bool mom = !wave && !ov && !sweep && !repair;  // moments inside the collision
       int tk = ov ? -1 : timer_begin(s);
       if (wave) {
         cudaMemsetAsync(f->wave_sync, 0, sizeof(int32_t) * (2 + 3 * (size_t)p->n_planes), s);
@@ -701,7 +701,7 @@ extern "C" int cvlbm3d_run(const cvlbm3d_problem* p, cvlbm3d_fields* f, double t
         k3_moments_part<1><<<blocks(p->n_link_nodes, 256), 256, 0, s>>>(
             c, f->f0, f->U, f->u_next, f->u_star, f->invalid, sweep);
         cv::count_launches(1);
-      } else if (N > 0) {
+      } else if (N > 0 && !mom) {
         k3_moments<<<blocks(N, 256), 256, 0, s>>>(c, f->f0, f->U, sweep ? f->u_next : f->u,
                                                   f->u_star, f->invalid, sweep);
         cv::count_launches(1);
@@ -711,8 +711,8 @@ extern "C" int cvlbm3d_run(const cvlbm3d_problem* p, cvlbm3d_fields* f, double t
           k3_sweep<<<blocks(N, 256), 256, 0, s>>>(c, f->U, f->u_next, f->u, f->u_star, clock, t);
           cv::count_launches(1);
         }
-        collide_fn<<<blocks(N, kCT3), kCT3, kCollideSmem3, s>>>(c, fz, f->f0, f->f1, f->U, f->u,
-                                                                repair, k == nsteps - 1);
+        (mom ? collide_mom : collide_fn)<<<blocks(N, kCT3), kCT3, kCollideSmem3, s>>>(
+            c, fz, f->f0, f->f1, f->U, f->u, repair, k == nsteps - 1, f->u, f->u_star, f->invalid);
         cv::count_launches(1);
         if (ov && k + 1 < nsteps) {
           // a sweep is due every step, so these moments write u_next

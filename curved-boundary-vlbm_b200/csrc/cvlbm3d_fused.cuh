@@ -423,17 +423,20 @@ __device__ __forceinline__ void collide_dir3(const Ctx3& c, const Fused3& fz,
 //    per direction (312 us) and rotating the state through registers (6 to 12 %).
 //
 // MAT >= 0: compiled for that material law.  MINB resident blocks per SM bound the
-// registers per thread.
+// registers per thread.  MOM (a step without sweep and repair): the moments are formed
+// here instead of by k3_moments; f0 then crosses HBM once per step and U only on the
+// last step (affine3d, 112^3: 57 + 128 us in two kernels).
 constexpr int kCT3 = 128;               // nodes per block
 constexpr int kCState3 = kC3 + 3 * 9;   // S (12), P(F) (9), change of P (9), change of F / 6 (9)
 
 constexpr int kCollideSmem3 = sizeof(double) * kCState3 * kCT3;
 
-template <int MAT, int MINB>
+template <int MAT, int MINB, bool MOM>
 __global__ void __launch_bounds__(kCT3, MINB)
     k3_collide(Ctx3 c, Fused3 fz, const double* __restrict__ f0, double* __restrict__ f1,
-                  double* __restrict__ U, const double* __restrict__ u, int do_repair,
-                  int store_all) {
+               double* __restrict__ U, const double* __restrict__ u, int do_repair,
+               int store_all, double* __restrict__ uw, double* __restrict__ ustar,
+               int* __restrict__ invalid) {
   extern __shared__ double sm3[];  // [kCState3][kCT3]; every thread uses its own column
   const int N = c.N, tid = threadIdx.x;
   const int n = blockIdx.x * kCT3 + tid;
@@ -449,7 +452,22 @@ __global__ void __launch_bounds__(kCT3, MINB)
   for (int q = 0; q < kQ3; ++q) nb[q] = p.neighbor[(size_t)q * N + n];
   const int slot = fz.need_slot[n];
   double S[kC3];
-  {
+  if constexpr (MOM) {
+    // neither sweep nor repair this step: the work of k3_moments, the collision's own
+    // reads of f0 below then come from L2
+    moments3(c, f0, n, S);
+    if (store_all) {
+#pragma unroll
+      for (int a = 0; a < kC3; ++a) U[(size_t)a * N + n] = S[a];
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double uu = ustar[(size_t)d * N + n] + c.hdt * S[d];
+      uw[(size_t)d * N + n] = uu;
+      ustar[(size_t)d * N + n] = uu + c.hdt * S[d];
+    }
+    if (det3(S[3], S[4], S[5], S[6], S[7], S[8], S[9], S[10], S[11]) <= c.m.jf) *invalid = 1;
+  } else {
     const double* src = U + n;
 #pragma unroll
     for (int a = 0; a < kC3; ++a) {
@@ -618,20 +636,21 @@ __global__ void __launch_bounds__(kCT3, MINB)
   }
 }
 
-using CollideFn3 = void (*)(Ctx3, Fused3, const double*, double*, double*, const double*, int, int);
+using CollideFn3 = void (*)(Ctx3, Fused3, const double*, double*, double*, const double*, int, int,
+                            double*, double*, int*);
 
 // The collision compiled for the problem's material law.
-template <int MINB>
+template <int MINB, bool MOM>
 CollideFn3 collide3(int model) {
   switch (model) {
-    case kMatSVK: return k3_collide<kMatSVK, MINB>;
-    case kMatNeoHooke: return k3_collide<kMatNeoHooke, MINB>;
-    case kMatLogNeoHooke: return k3_collide<kMatLogNeoHooke, MINB>;
-    case kMatMooneyRivlin: return k3_collide<kMatMooneyRivlin, MINB>;
-    case kMatYeoh: return k3_collide<kMatYeoh, MINB>;
-    case kMatGent: return k3_collide<kMatGent, MINB>;
-    case kMatSix: return k3_collide<kMatSix, MINB>;
-    default: return k3_collide<-1, MINB>;
+    case kMatSVK: return k3_collide<kMatSVK, MINB, MOM>;
+    case kMatNeoHooke: return k3_collide<kMatNeoHooke, MINB, MOM>;
+    case kMatLogNeoHooke: return k3_collide<kMatLogNeoHooke, MINB, MOM>;
+    case kMatMooneyRivlin: return k3_collide<kMatMooneyRivlin, MINB, MOM>;
+    case kMatYeoh: return k3_collide<kMatYeoh, MINB, MOM>;
+    case kMatGent: return k3_collide<kMatGent, MINB, MOM>;
+    case kMatSix: return k3_collide<kMatSix, MINB, MOM>;
+    default: return k3_collide<-1, MINB, MOM>;
   }
 }
 
@@ -858,12 +877,55 @@ __global__ void __launch_bounds__(128)
     for (int k = 0; k < 4; ++k) char_state[((size_t)k * 12 + a0 + cc) * L + ell] = acc[cc][k];
 }
 
+// F predictor of the link from U at the node and its upstream node (BFL and
+// compat_bfl reconstructions, :2887-2990), tangential image from the LSQ stencil.
+static __device__ __noinline__ void predictor3(const Ctx3& c, const Fused3& fz, int ell,
+                                               const double* u, double* F) {
+  const cvlbm3d_problem& p = c.p;
+  const int N = c.N, n = p.link_p[ell], upid = p.link_up[ell];
+  const double eta = p.link_eta[ell];
+  const double* Un = fz.Uneed + (size_t)fz.need_slot[n] * kC3;
+  for (int k = 0; k < 9; ++k) F[k] = Un[3 + k];
+  if (!(p.recon == 2 || p.recon == 4)) return;
+  if (upid >= 0) {
+    const double* Uu = fz.Uneed + (size_t)fz.need_slot[upid] * kC3;
+    for (int k = 0; k < 9; ++k) F[k] = Un[3 + k] + eta * (Un[3 + k] - Uu[3 + k]);
+  }
+  if (p.recon == 2 && p.has_tangent_lsq && p.lsq_valid[ell] != 0) {
+    Frame3 fr = frame3(p.link_nx[ell], p.link_ny[ell], p.link_nz[ell]);
+    double du1[3] = {0, 0, 0}, du2[3] = {0, 0, 0}, wt_abs = 0.0;
+    for (int mm = 0; mm < kMaxLsq3; ++mm) {
+      const int q = p.lsq_p[(size_t)ell * kMaxLsq3 + mm];
+      if (q >= 0) {
+        const double w1 = p.lsq_wt1[(size_t)ell * kMaxLsq3 + mm];
+        const double w2 = p.lsq_wt2[(size_t)ell * kMaxLsq3 + mm];
+        for (int r = 0; r < 3; ++r) {
+          du1[r] += w1 * u[(size_t)r * N + q];
+          du2[r] += w2 * u[(size_t)r * N + q];
+        }
+        wt_abs += fabs(w1) + fabs(w2);
+      }
+    }
+    if (wt_abs > 0.0) {
+      double h[3], g1[3], g2[3];
+      for (int r = 0; r < 3; ++r) {
+        h[r] = F[3 * r] * fr.n[0] + F[3 * r + 1] * fr.n[1] + F[3 * r + 2] * fr.n[2];
+        g1[r] = fr.t1[r] + du1[r];
+        g2[r] = fr.t2[r] + du2[r];
+      }
+      for (int r = 0; r < 3; ++r)
+        for (int s = 0; s < 3; ++s)
+          F[3 * r + s] = h[r] * fr.n[s] + g1[r] * fr.t1[s] + g2[r] * fr.t2[s];
+    }
+  }
+}
+
 // Boundary value, F predictor, Newton normal solve and P(F_b) of one link;
 // the results go to the link buffers (link_kind .. link_Pb), which the
 // reference also exposes (three_d/curved_boundary_warp3d.py:4281-4337).
 __global__ void __launch_bounds__(128)
-    k3_link_prepare(Ctx3 c, Fused3 fz, const double* __restrict__ u, cvlbm3d_fields fl,
-                    const double* clock, double t_host, double offset) {
+    k3_link_prepare(const __grid_constant__ Ctx3 c, const __grid_constant__ Fused3 fz,
+                    const double* __restrict__ u, cvlbm3d_fields fl, const double* clock, double t_host, double offset) {
   const cvlbm3d_problem& p = c.p;
   const Mat& m = c.m;
   const int L = p.n_links, N = c.N;
@@ -889,42 +951,8 @@ __global__ void __launch_bounds__(128)
   double Pb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   const bool anyN = ck[0] == kNeumann || ck[1] == kNeumann || ck[2] == kNeumann;
   if (anyN) {
-    const double* Un = fz.Uneed + (size_t)fz.need_slot[n] * kC3;
     double F[9];
-    for (int k = 0; k < 9; ++k) F[k] = Un[3 + k];
-    if (p.recon == 2 || p.recon == 4) {
-      if (upid >= 0) {
-        const double* Uu = fz.Uneed + (size_t)fz.need_slot[upid] * kC3;
-        for (int k = 0; k < 9; ++k) F[k] = Un[3 + k] + eta * (Un[3 + k] - Uu[3 + k]);
-      }
-      if (p.recon == 2 && p.has_tangent_lsq && p.lsq_valid[ell] != 0) {
-        Frame3 fr = frame3(nx, ny, nz);
-        double du1[3] = {0, 0, 0}, du2[3] = {0, 0, 0}, wt_abs = 0.0;
-        for (int mm = 0; mm < kMaxLsq3; ++mm) {
-          const int q = p.lsq_p[(size_t)ell * kMaxLsq3 + mm];
-          if (q >= 0) {
-            const double w1 = p.lsq_wt1[(size_t)ell * kMaxLsq3 + mm];
-            const double w2 = p.lsq_wt2[(size_t)ell * kMaxLsq3 + mm];
-            for (int r = 0; r < 3; ++r) {
-              du1[r] += w1 * u[(size_t)r * N + q];
-              du2[r] += w2 * u[(size_t)r * N + q];
-            }
-            wt_abs += fabs(w1) + fabs(w2);
-          }
-        }
-        if (wt_abs > 0.0) {
-          double h[3], g1[3], g2[3];
-          for (int r = 0; r < 3; ++r) {
-            h[r] = F[3 * r] * fr.n[0] + F[3 * r + 1] * fr.n[1] + F[3 * r + 2] * fr.n[2];
-            g1[r] = fr.t1[r] + du1[r];
-            g2[r] = fr.t2[r] + du2[r];
-          }
-          for (int r = 0; r < 3; ++r)
-            for (int s = 0; s < 3; ++s)
-              F[3 * r + s] = h[r] * fr.n[s] + g1[r] * fr.t1[s] + g2[r] * fr.t2[s];
-        }
-      }
-    }
+    if (p.recon != 3) predictor3(c, fz, ell, u, F);
     if (p.recon == 3 && p.has_char && p.char_idx[ell] >= 0)
       for (int k = 0; k < 9; ++k) F[k] = fl.char_state[((size_t)0 * 12 + 3 + k) * L + ell];
     else if (p.recon == 3)

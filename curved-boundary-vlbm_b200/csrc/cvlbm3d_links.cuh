@@ -152,8 +152,15 @@ __global__ void __launch_bounds__(kFinish3, 6)
   }
   if (anyN) {
     double F[9];
+    if (p.recon == 3) {
 #pragma unroll
-    for (int k = 0; k < 9; ++k) F[k] = gathered ? cs[(size_t)(3 + k) * L] : 0.0;
+      for (int k = 0; k < 9; ++k) F[k] = gathered ? cs[(size_t)(3 + k) * L] : 0.0;
+    } else {
+      double F2[9];
+      predictor3(c, fz, ell, u, F2);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) F[k] = F2[k];
+    }
 #pragma unroll
     for (int k = 0; k < 9; ++k) Fb[k] = F[k];
     if (ck[0] == kNeumann && ck[1] == kNeumann && ck[2] == kNeumann)
