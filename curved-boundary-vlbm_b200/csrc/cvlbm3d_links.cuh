@@ -14,6 +14,10 @@
 // solver sat in one kernel.  One kernel with four lanes per link for everything
 // (tangents and evaluations of P spread over the lanes) was 50 us and 498 us: it
 // repeats the normal solve on every lane.
+// Four lanes per link in k3_link_finish alone (three tangents and P at the state side
+// by side) cost 1 us per step more at 3,920 to 11,256 links, 8 at 15,448 and 20 at
+// 25,320: the chain's length there is the unique code a warp runs through, not the
+// number of tangents.
 #pragma once
 
 namespace {

@@ -54,9 +54,11 @@ struct Mat {
 // against it by the tests - at four FP64 operations instead of a reciprocal
 // sequence, range checks and branches per division: the D2Q4 node kernel makes
 // about 20 such divisions per node and the D3Q6 one 29.  Outside a safe range
-// of exponents (and for infinities and NaN) the division itself runs.  A quotient
-// below about 1e-270 may differ in its last place (the remainder is subnormal);
-// every kernel forms its quotients here, so they agree with one another.
+// of exponents (divc: of either operand, infinities and NaN included; div_n: of the
+// divisor) the division itself runs.  A quotient below about 1e-270 may differ in
+// its last place (the remainder is subnormal), and div_n of a numerator above 2^900,
+// which only a diverged state has, may give NaN for an infinity; every kernel forms
+// its quotients here, so they agree with one another.
 // ---------------------------------------------------------------------------
 CV_DEV uint32_t mag_hi(double a) { return (uint32_t)__double2hiint(a) & 0x7fffffffu; }
 
