@@ -595,15 +595,26 @@ class WarpCurvedBoundaryLBM2D:
                 if int(self._lib.cvlbm2d_tile_variant(int(v))) > 0]
         times = {}
         # timed as run() will execute it: a graph replay for even counts (launched one by
-        # one, the small kernels of a step are bound by the launches, whatever the tile)
+        # one, the small kernels of a step are bound by the launches, whatever the tile);
+        # short graphs, because capturing one costs more than replaying it.  Where a
+        # graph of that length would not fit the next steps (its kinematic phase
+        # differs) the launches are timed.
+        steps = int(steps)
+        short = self.GRAPH_MIN_STEPS
+        replay = steps % short == 0 and all(
+            short % iv == 0 for iv in (self.local_displacement_interval,
+                                       self.local_compatibility_interval) if iv > 0)
+        chunk = short if replay else steps
+        use_graphs, self.use_graphs = self.use_graphs, self.use_graphs and replay
         for v in cand:
             self._select_variant(v)
             self._graphs.clear()
-            self.run(steps)
+            self.run(chunk)
             torch.cuda.synchronize(self._tdev)
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
-            self.run(steps)
+            for _ in range(steps // chunk):
+                self.run(chunk)
             e1.record()
             e1.synchronize()
             times[v] = e0.elapsed_time(e1) * 1e3 / steps
@@ -611,6 +622,7 @@ class WarpCurvedBoundaryLBM2D:
             self.U.copy_(saved[3]); self.u.copy_(saved[4])
             self.time, self.steps = saved[5], saved[6]
         self._graphs.clear()
+        self.use_graphs = use_graphs
         best = min(times, key=times.get)
         self._select_variant(best)
         return times
