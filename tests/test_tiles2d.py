@@ -79,3 +79,17 @@ def test_batch_runs_the_staged_tiles_and_refuses_the_others():
     for v in (5, 6, 7, 11):
         with pytest.raises((RuntimeError, ValueError)):
             BatchedCurvedBoundaryLBM2D([_solver(40)], tile_variant=v)
+
+
+@pytest.mark.parametrize("steps,kw", [(16, {}), (10, {}), (16, {"local_displacement_interval": 3}),
+                                      (5, {})])
+def test_autotune_replays_or_launches_and_restores_the_state(steps, kw):
+    s = _solver(64, **kw)
+    s.run(1)
+    before = [s.numpy_field(k) for k in ("f0", "u_star")], s.time, s.steps
+    times = s.autotune(steps=steps)
+    assert len(times) == 11 and min(times.values()) > 0 and s.tile_variant in times
+    assert s.use_graphs and not s._graphs
+    assert (s.time, s.steps) == before[1:]
+    for a, b in zip(before[0], (s.numpy_field("f0"), s.numpy_field("u_star"))):
+        assert np.array_equal(a, b)
