@@ -28,10 +28,16 @@ import time as _time
 import numpy as np
 
 from . import _native
-from .two_d.curved_boundary_warp import DEFAULT_TILE_VARIANT
 
 BATCH_VARIANTS = (0, 1, 2, 3, 4, 8, 9, 10)  # tile shapes a batch can run
 BATCH_DEFAULT_VARIANT = 8
+
+
+def batch_tile_variant(solver) -> int:
+    """The solver's tile shape if it was tuned or selected and a batch can run it, else the
+    staged 8 x 32 tile (24 shells: 223 us per step against 253 with the solvers' default)."""
+    chosen = solver._tile_variant_chosen and solver.tile_variant in BATCH_VARIANTS
+    return int(solver.tile_variant) if chosen else BATCH_DEFAULT_VARIANT
 
 
 class BatchedCurvedBoundaryLBM2D:
@@ -58,11 +64,7 @@ class BatchedCurvedBoundaryLBM2D:
         self._lib = _native.load()
         self.grid_blocks = int(grid_blocks)
         if tile_variant is None:
-            # the solvers' shape if it was chosen for them, else the staged 8 x 32 tile
-            # (24 shells: 223 us per step against 253 with the solvers' default)
-            tile_variant = self.solvers[0].tile_variant
-            if tile_variant == DEFAULT_TILE_VARIANT or int(tile_variant) not in BATCH_VARIANTS:
-                tile_variant = BATCH_DEFAULT_VARIANT
+            tile_variant = batch_tile_variant(self.solvers[0])
         self.tile_variant = int(tile_variant)
         self.handle = None
         self._graphs: dict = {}

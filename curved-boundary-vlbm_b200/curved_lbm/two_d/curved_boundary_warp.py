@@ -540,6 +540,7 @@ class WarpCurvedBoundaryLBM2D:
         sms = torch.cuda.get_device_properties(self._tdev).multi_processor_count
         if self._problem.n_tiles > DEFAULT_TILES_PER_SM * sms:
             self._select_variant(DEFAULT_TILE_VARIANT_LARGE)
+        self._tile_variant_chosen = False  # so far the default; a batch picks its own then
         self.initialize_identity(init_order=1)
 
     # -- native plumbing ---------------------------------------------------
@@ -573,6 +574,7 @@ class WarpCurvedBoundaryLBM2D:
         tiles, tj, n_inner = self._tile_lists[tile_i]
         self._tables["tiles"] = tiles
         self.tile_variant = int(variant)
+        self._tile_variant_chosen = True
         p = self._problem
         p.tile_variant, p.tile_i = int(variant), tile_i
         p.n_tiles, p.tiles_j = int(tiles.numel()), int(tj)
