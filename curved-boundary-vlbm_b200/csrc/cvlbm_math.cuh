@@ -15,12 +15,6 @@
 
 #define CV_DEV __device__ __forceinline__
 
-#ifdef DIVI
-#define DIVF(a, b) ((a) / (b))
-#endif
-#ifndef DIVF
-#define DIVF div_ieee
-#endif
 namespace cv {
 
 constexpr double kPi = 3.141592653589793238462643383279502884;
@@ -50,16 +44,30 @@ struct Mat {
 // q = RN(a y + RN(a e)) is a faithful quotient, its remainder a - b q is exact in
 // one FMA, and RN(q + (a - b q) y) is the correctly rounded a/b (Markstein 1990,
 // theorem on a faithful q and a correctly rounded reciprocal; Brisebarre, Muller
-// and Raina 2004 for known divisors).  The bits are those of a / b - checked
-// against it by the tests - at four FP64 operations instead of a reciprocal
+// and Raina 2004 for known divisors).  Four FP64 operations instead of a reciprocal
 // sequence, range checks and branches per division: the D2Q4 node kernel makes
-// about 20 such divisions per node and the D3Q6 one 29.  Outside a safe range
-// of exponents (divc: of either operand, infinities and NaN included; div_n: of the
-// divisor) the division itself runs.  A quotient below about 1e-270 may differ in
-// its last place (the remainder is subnormal), and div_n of a numerator above 2^900,
-// which only a diverged state has, may give NaN for an infinity; every kernel forms
-// its quotients here, so they agree with one another.
+// about 20 such divisions per node and the D3Q6 one 29.
+//
+// The short form runs for a divisor in 2^-100 .. 2^100 and numerators below 2^900;
+// otherwise (infinities and NaN among them) the division itself does, for all
+// numerators of a group if one is out of range.  Where the short form runs, the
+// quotient of a numerator of at least 2^-968 has the bits of a / b, checked by the
+// tests on the device.  Two exceptions:
+//  * a zero numerator gives a zero, but its sign can be the other one than that of
+//    a / b (+0 for -0 / 3): the sums above lose it.  Nothing here reads that sign, and
+//    the two compare equal.  Putting it back from the numerator lengthened the links'
+//    and nodes' chains by 0.8 to 2.2 % of a step (4,505 to 4,623 us for 50 steps of a
+//    tube on 48 x 48 x 96 nodes).
+//  * a smaller nonzero numerator has a remainder that rounds on the subnormal grid:
+//    its quotient is within two units in the last place.
+// The range check stands behind the quotients, so that it runs beside them: before
+// them it added 1 to 4 % to a step, behind them nothing (1,083 us against 1,087 without
+// a check of the numerators, 701^2 Mooney-Rivlin).
 // ---------------------------------------------------------------------------
+constexpr uint32_t kQuotLo = 0x39b00000u;   // high word of 2^-100
+constexpr uint32_t kQuotHi = 0x46300000u;   // of 2^100
+constexpr uint32_t kQuotNum = 0x78300000u;  // of 2^900
+
 CV_DEV uint32_t mag_hi(double a) { return (uint32_t)__double2hiint(a) & 0x7fffffffu; }
 
 CV_DEV double quot(double a, double b, double y, double e) {
@@ -79,7 +87,7 @@ inline DivC make_divc(double b) {
   d.y = 1.0 / b;
   d.e = ::fma(-b, d.y, 1.0) * d.y;
   const double m = ::fabs(b);
-  d.lim = (m >= 7.9e-31 && m <= 1.2e30) ? 0x78300000u : 0u;  // 2^-100 .. 2^100; |a| < 2^900
+  d.lim = (m >= 0x1p-100 && m < 0x1p100) ? kQuotNum : 0u;
   return d;
 }
 
@@ -89,13 +97,13 @@ inline DivC make_divc(double b) {
 static __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
 
 CV_DEV double divc(double a, const DivC& d) {
-  if (mag_hi(a) < d.lim) return quot(a, d.b, d.y, d.e);
-  return DIVF(a, d.b);
+  double q = quot(a, d.b, d.y, d.e);
+  if (mag_hi(a) >= d.lim) q = div_ieee(a, d.b);
+  return q;
 }
 
-// A divisor formed in the kernel, shared by several numerators of moderate size
-// (cofactors over their determinant, differences over a step): the short form is
-// used when the divisor lies in 2^-100 .. 2^100.
+// A divisor formed in the kernel, shared by several numerators (cofactors over their
+// determinant, differences over a step).
 struct Rcp {
   double b, y, e;
   bool ok;
@@ -106,17 +114,21 @@ CV_DEV Rcp rcp_of(double b) {
   r.b = b;
   r.y = 1.0 / b;
   r.e = fma(-b, r.y, 1.0) * r.y;
-  r.ok = mag_hi(b) - 0x39b00000u < 0x46300000u - 0x39b00000u;
+  r.ok = mag_hi(b) - kQuotLo < kQuotHi - kQuotLo;
   return r;
 }
 
+// out[k] = a[k] / r.b, n a constant of the caller
 CV_DEV void div_n(const Rcp& r, const double* a, double* out, int n) {
-  if (r.ok) {
+  uint32_t top = 0;
 #pragma unroll
-    for (int k = 0; k < n; ++k) out[k] = quot(a[k], r.b, r.y, r.e);
-  } else {
+  for (int k = 0; k < n; ++k) {
+    top = max(top, mag_hi(a[k]));
+    out[k] = quot(a[k], r.b, r.y, r.e);
+  }
+  if (!r.ok || top >= kQuotNum) {
 #pragma unroll
-    for (int k = 0; k < n; ++k) out[k] = DIVF(a[k], r.b);
+    for (int k = 0; k < n; ++k) out[k] = div_ieee(a[k], r.b);
   }
 }
 
