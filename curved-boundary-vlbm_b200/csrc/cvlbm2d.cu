@@ -722,8 +722,17 @@ FusedLaunch2 fused_variant(int v, int model = -1) {
   return model == kMatNeoHooke ? fused_variant_as<kMatNeoHooke>(v) : fused_variant_as<-1>(v);
 }
 
+// Numbers 6 and 7 once stood for shapes of 16 and 8 rows.  A problem that carries one of
+// them with a tile list of that height runs the shape of that height (results are the
+// same bits) instead of the per-phase kernels: 40 against 96 us per step at 512^2.
+int shape_of(const cvlbm2d_problem* p) {
+  if (p->tile_variant == 6 && p->tile_i == 16) return 0;
+  if (p->tile_variant == 7 && p->tile_i == 8) return 2;
+  return p->tile_variant;
+}
+
 bool fused_ok(const cvlbm2d_problem* p, const cvlbm2d_fields* f) {
-  const FusedLaunch2 fl = fused_variant(p->tile_variant);
+  const FusedLaunch2 fl = fused_variant(shape_of(p));
   return p->tiles && p->need_fields && p->link_partner && f->link_scratch && p->lsq_node &&
          p->disp_sweeps <= 1 && fl.tile_i == p->tile_i &&
          p->collision_model == 0 && !(p->kinetic_filter > 0.0) &&
@@ -746,7 +755,7 @@ extern "C" int cvlbm2d_run(const cvlbm2d_problem* p, cvlbm2d_fields* f, double t
   k_zero_flag<<<1, 1, 0, s>>>(f->invalid); cv::count_launches(1);
   double t = time0;
   const bool fused = fused_ok(p, f);
-  FusedLaunch2 fl = fused_variant(p->tile_variant, p->mat.model);
+  FusedLaunch2 fl = fused_variant(shape_of(p), p->mat.model);
   const bool split = fused && p->tile_variant == kSplitVariant;
   if (fused && !split)
     cudaFuncSetAttribute(fl.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fl.smem);

@@ -140,7 +140,9 @@ typedef struct cvlbm2d_problem {
 } cvlbm2d_problem;
 
 /* Tile rows (i extent, tiles are 32 nodes wide in j) of fused-kernel variant
- * v, or 0 if v is not compiled.  Used by autotuners to enumerate variants. */
+ * v, or 0 if v is not compiled.  Used by autotuners to enumerate variants.
+ * Variants 6 and 7 have 10 and 9 rows; they once had 16 and 8, and a problem
+ * whose tile list has those (`tile_i`) runs variant 0 or 2 instead. */
 int cvlbm2d_tile_variant(int32_t v);
 
 /* Mutable state.  f0 is the current population field; a run swaps f0 and f1
