@@ -250,15 +250,15 @@ __global__ void __launch_bounds__(128)
 // of later slices while another has the MMAs of slice k in flight; stage s is
 // refilled once the MMAs that read it have committed to empty[s].
 //
-// Tile width BN and stages ST (launch rule in launch_tma):
+// Tile width BN (64 or 128) and stages ST (launch rule in cvlbm_gemm_bf16):
 //  * BN = 128, ST = 3 (97 KB): two CTAs per SM.
 //  * BN = 128, ST = 2 (65 KB): three CTAs per SM, taken when the grid then fits one
 //    wave (the forward transform of the 32 x 32 x 64 lattice: 384 CTAs).
 //  * Few CTAs (a K that does not split): BN = 64 with six stages.  The CTA is then
 //    bound by its chain of dependent MMAs (one 16-deep step of K after the other
-//    into the same accumulators, about 78 ns each at N = 64 or 32, 100 ns at 128):
-//    128 x 768 x 93312 in two splits 228 us against 291; narrower tiles and more
-//    stages measured the same.  Every element sums its K range in the same order.
+//    into the same accumulators, about 78 ns each at N = 64, 100 ns at 128):
+//    128 x 768 x 93312 in two splits, 24 CTAs, 228 us against 291 in 12; tiles of
+//    32 columns and more stages measured the same.  Every element sums its K range in the same order.
 //
 // Shared-memory descriptor of a SWIZZLE_128B K-major tile: start address,
 // stride between 8-row atoms 1024 bytes, leading offset unused (1), version
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(128)
     // A lane storing 16 bytes of its own row touched 32 lines per instruction,
     // and with `accumulate` waited for each such load before the next: 150 us
     // against 40 us at 128 x 65536 x 768.
-    constexpr int CW = BN < 64 ? BN : 64, LD = CW + 4, LPR = CW / 4, RPI = 32 / LPR, IT = 32 / RPI;
+    constexpr int CW = 64, LD = CW + 4, LPR = CW / 4, RPI = 32 / LPR, IT = 32 / RPI;
     float* st = reinterpret_cast<float*>(smem_t + (base - smem_u32(smem_t))) + warp * 32 * LD;
     const int row0 = m0 + warp * 32;
     float* dst0 = partial ? partial + (size_t)blockIdx.z * M * N + (size_t)row0 * N + n0
@@ -502,7 +502,7 @@ template <int BN, int ST>
 void launch_tma_as(dim3 grid, cudaStream_t s, const CUtensorMap& a, const CUtensorMap& b, float* C,
                    float* part, int M, int N, int kchunk, int ldc, int accumulate, int* error) {
   constexpr int smem = ST * (kBM + BN) * kBK * 2 + 1024;
-  static_assert(smem - 1024 >= kBM * ((BN < 64 ? BN : 64) + 4) * 4, "epilogue staging");
+  static_assert(smem - 1024 >= kBM * (64 + 4) * 4, "epilogue staging");
   cudaFuncSetAttribute(k_gemm_tma<BN, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   k_gemm_tma<BN, ST><<<grid, 128, smem, s>>>(a, b, C, part, M, N, kchunk, ldc, accumulate, error);
 }
