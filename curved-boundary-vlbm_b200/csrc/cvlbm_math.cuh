@@ -60,9 +60,8 @@ struct Mat {
 //    tube on 48 x 48 x 96 nodes).
 //  * a smaller nonzero numerator has a remainder that rounds on the subnormal grid:
 //    its quotient is within two units in the last place.
-// The range check stands behind the quotients, so that it runs beside them: before
-// them it added 1 to 4 % to a step, behind them nothing (1,083 us against 1,087 without
-// a check of the numerators, 701^2 Mooney-Rivlin).
+// With the range check the measured steps take what they took without a check of the
+// numerators (where it stands: div_n).
 // ---------------------------------------------------------------------------
 constexpr uint32_t kQuotLo = 0x39b00000u;   // high word of 2^-100
 constexpr uint32_t kQuotHi = 0x46300000u;   // of 2^100
@@ -118,17 +117,24 @@ CV_DEV Rcp rcp_of(double b) {
   return r;
 }
 
-// out[k] = a[k] / r.b, n a constant of the caller
+// out[k] = a[k] / r.b, n a constant of the caller.  Small groups form the quotients and
+// check the numerators beside them; nine cofactors do not stay in registers beside their
+// quotients, so their check comes first, hidden behind the reciprocal (112^3 affine, four
+// steps: 783 us, 789 with the check behind; 701^2 Mooney-Rivlin, groups of four: 1,091 and
+// 1,084).
 CV_DEV void div_n(const Rcp& r, const double* a, double* out, int n) {
   uint32_t top = 0;
 #pragma unroll
   for (int k = 0; k < n; ++k) {
     top = max(top, mag_hi(a[k]));
-    out[k] = quot(a[k], r.b, r.y, r.e);
+    if (n < 9) out[k] = quot(a[k], r.b, r.y, r.e);
   }
   if (!r.ok || top >= kQuotNum) {
 #pragma unroll
     for (int k = 0; k < n; ++k) out[k] = div_ieee(a[k], r.b);
+  } else if (n >= 9) {
+#pragma unroll
+    for (int k = 0; k < n; ++k) out[k] = quot(a[k], r.b, r.y, r.e);
   }
 }
 
