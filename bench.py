@@ -350,15 +350,20 @@ def measured_peaks():
     return {"hbm_gbs": HBM_FALLBACK_GBS}, "fallback"
 
 
-def ncu_traffic(workload: str):
+def ncu_traffic(workload: str, tile_variant=None):
     """(DRAM bytes per launch of the bracketed node kernels, where they come from),
-    read from the committed ncu summary figures."""
+    read from the committed ncu summary figures; of the tile shape that runs where the
+    figures are per shape."""
     path = ROOT / "profiles" / "traffic.json"
     if not path.exists():
         return None, None
     try:
         ent = json.loads(path.read_text()).get(workload) or {}
-        return ent.get("bytes"), ent.get("source")
+        by_shape = ent.get("bytes_by_tile_variant")
+        if by_shape is None:
+            return ent.get("bytes"), ent.get("source")
+        found = by_shape.get(str(tile_variant))
+        return found, ent.get("source") if found is not None else None
     except Exception:
         return None, None
 
@@ -695,7 +700,7 @@ def main():
     avg_kern_s = kern_ms * 1e-3 / max(kern_n, 1)
     algo_bytes = n_active * BYTES_PER_UPDATE[args.workload]
     achieved = algo_bytes / avg_kern_s / 1e9 if kern_n else None
-    traffic, traffic_src = ncu_traffic(args.workload)
+    traffic, traffic_src = ncu_traffic(args.workload, getattr(solver, "tile_variant", None))
     roofline = {"bound": "hbm", "kernel": "bulk node kernel (bracketed per lattice step)",
                 "achieved": achieved, "peak": peaks.get("hbm_gbs", HBM_FALLBACK_GBS),
                 "peak_kind": peak_kind, "unit": "GB/s",

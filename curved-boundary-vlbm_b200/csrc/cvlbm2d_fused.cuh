@@ -8,8 +8,9 @@
 // the first halo node's loads go with the node's own where the registers allow it,
 // nodes with four neighbours take straight-line code in the sweep and the repair, and
 // a population is stored through a pointer and a stride per direction instead of a
-// branch per component.  Per step, launches one by one: 100^2 29 to 25 us, 512^2 51
-// to 40, 701^2 74 to 60 (Mooney-Rivlin 114 to 92), affine 384^2 33 to 25.
+// branch per component.  Per step with the default shapes, launches one by one: 100^2
+// 29 to 24 us, 512^2 51 to 37, 701^2 74 to 53 (Mooney-Rivlin 114 to 68), affine 384^2 33
+// to 23; replayed from a graph 20, 34, 51, 68 and 20 us.
 //   A  every node of the tile plus a 3-node halo: moments and collide-time
 //      displacement u from f0, u* into shared memory (halo moments are
 //      recomputed from f0 through L2 instead of being exchanged);

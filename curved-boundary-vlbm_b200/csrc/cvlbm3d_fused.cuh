@@ -192,7 +192,8 @@ __device__ __forceinline__ void sweep_node3(const Ctx3& c, const double* U, cons
     }
   };
   if ((nb[0] | nb[1] | nb[2] | nb[3] | nb[4] | nb[5]) >= 0) {
-    // all six neighbours: their 36 values are loaded before the first is used
+    // all six neighbours: no load waits for a sum; the kernel's 64 registers hold only part
+    // of the 36 values at once
     double e[kQ3][3], un[kQ3][3];
 #pragma unroll
     for (int q = 0; q < kQ3; ++q) {

@@ -369,7 +369,7 @@ typedef struct cvlbm3d_problem {
                                                      and char_w_lm holds per link and slot
                                                      m < 48 the three gradient weights and,
                                                      for m < 16, the value weight of slot
-                                                     48 + m (else 0): one kernel then does
+                                                     48 + m (else 0): two kernels then do
                                                      all link work of a step */
   int32_t reserved0;
 } cvlbm3d_problem;
